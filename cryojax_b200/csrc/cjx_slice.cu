@@ -112,19 +112,16 @@ __global__ void __launch_bounds__(kWarps * 32)
 // half-plane slice H[kx][ky] to an L2-resident buffer, then a column kernel
 // that runs the Hermitian fix, inverse FFT and window on H.
 // ---------------------------------------------------------------------------
-// Minimum resident CTAs per SM the compiler must allow for (register cap).
-#ifndef CJX_GATHER_MIN_BLOCKS
-#define CJX_GATHER_MIN_BLOCKS 1
-#endif
-
-// Spline instances: 64 taps per sample would take ~170 registers if every
-// load were hoisted; two resident CTAs per SM cap them at 128.
-#ifndef CJX_SPLINE_MIN_BLOCKS
-#define CJX_SPLINE_MIN_BLOCKS 2
-#endif
+// Resident CTAs per SM that the split gather must allow for (register cap).
+// Trilinear instances of one or two samples per lane: 4 (64 registers; at the
+// 71 that the compiler takes without the cap, 3 fit and N = 360 took 0.40 ms per
+// 512 images instead of 0.35).  Spline instances: 64 taps per sample would take
+// about 170 registers if every load were hoisted; 2 CTAs cap them at 128.
+template <int S, typename Layout>
+constexpr int kGatherCtas = is_spline_layout<Layout>::value ? 2 : (S <= 2 ? 4 : 1);
 
 template <int S, typename Layout, int MAP>
-__global__ void __launch_bounds__(256, is_spline_layout<Layout>::value ? CJX_SPLINE_MIN_BLOCKS : CJX_GATHER_MIN_BLOCKS)
+__global__ void __launch_bounds__(256, (kGatherCtas<S, Layout>))
     k_gather_slice(const float2* __restrict__ grid, const cjx_image_params* __restrict__ params,
                    const int32_t* __restrict__ order, float2* __restrict__ hbuf, SliceGeom g, int64_t k0) {
   const Layout L(g.n);
@@ -175,6 +172,83 @@ __global__ void __launch_bounds__(256, is_spline_layout<Layout>::value ? CJX_SPL
 #pragma unroll
   for (int s = 0; s < S; ++s)
     if (act[s]) col[vbase + 16 * s] = val[s];
+}
+
+// The split gather for spline coefficients in the x-pair layout, four lanes
+// per sample (sample_spline_team4), bound by the L1's data stage (77 % of its
+// wavefronts, ncu) next to the issue slots (65 %).  512 images 320^2 from
+// N = 512: 3.13 ms with a lane per sample, 2.48 ms now; with 2, 3, 4 and 5
+// CTAs per SM 3.30, 2.70, 2.48 and 2.98 ms (5 spill).  A warp takes 4 columns x 8 rows as four groups of 2 x 4 samples;
+// the four lanes of a team then exchange their shares, so that lane t ends
+// with the sample of group t, and store it.
+// CTA patch: 16 columns x 16 kSplineSteps rows.
+constexpr int kSplineSteps = 4;
+
+__global__ void __launch_bounds__(256, 4)
+    k_gather_spline_team(const float4* __restrict__ coef, const cjx_image_params* __restrict__ params,
+                         const int32_t* __restrict__ order, float2* __restrict__ hbuf, SliceGeom g, int64_t k0) {
+  const SplinePairLayout L(g.n);
+  const int n = g.n;
+  const int64_t k = k0 + blockIdx.z;
+  const int64_t img = order ? (int64_t)order[k] : k;
+  const double* R = params[img].rot;
+  const float r00 = (float)R[0], r01 = (float)R[1];
+  const float r10 = (float)R[3], r11 = (float)R[4];
+  const float r20 = (float)R[6], r21 = (float)R[7];
+  const bool ewald = (g.flags & CJX_EWALD_SPHERE) != 0;
+  float cw = 0.f, r02 = 0.f, r12 = 0.f, r22 = 0.f;
+  if (ewald) {
+    cw = ewald_w(params + img, n);
+    r02 = (float)R[2];
+    r12 = (float)R[5];
+    r22 = (float)R[8];
+  }
+  const bool wrap = !(g.flags & CJX_ZERO_FILL_NEGATIVE);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t = lane & 3, ly = t & 1, lz = t >> 1;
+  const int su = (lane >> 2) & 1, sv = lane >> 3;
+  const int u0 = blockIdx.x * 16 + 4 * (warp & 3);
+  float ux[2], bx[2], by[2], bz[2];  // the two columns this lane samples
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    ux[c] = (float)fft_index(min(u0 + 2 * c + su, n - 1), n);
+    bx[c] = r00 * ux[c];
+    by[c] = r10 * ux[c];
+    bz[c] = r20 * ux[c];
+  }
+#pragma unroll 1
+  for (int step = 0; step < kSplineSteps; ++step) {
+    const int v0 = (blockIdx.y * kSplineSteps + step) * 16 + 8 * (warp >> 2);
+    if (v0 >= n) break;  // the same for the whole warp
+    float2 p[4];
+    // every lane samples (columns and rows past the edge repeat others); only the stores are guarded
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int c = q & 1;
+      const float v = (float)(v0 + sv) + 4.0f * (q >> 1);
+      const float vy = v < (float)(n - n / 2) ? v : v - (float)n;  // fft_index of the row
+      float ox = fmaf(r01, vy, bx[c]), oy = fmaf(r11, vy, by[c]), oz = fmaf(r21, vy, bz[c]);
+      if (ewald) {
+        const float w = cw * fmaf(ux[c], ux[c], vy * vy);
+        ox = fmaf(r02, w, ox);
+        oy = fmaf(r12, w, oy);
+        oz = fmaf(r22, w, oz);
+      }
+      p[q] = sample_spline_team4(coef, n, L, ox, oy, oz, wrap, g.fill, ly, lz);
+    }
+    float2 s[2];  // groups ly and ly + 2, summed over ly
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const float2 give = ly ? p[2 * c] : p[2 * c + 1], own = ly ? p[2 * c + 1] : p[2 * c];
+      s[c] = __fadd2_rn(own, make_float2(__shfl_xor_sync(0xffffffffu, give.x, 1),
+                                         __shfl_xor_sync(0xffffffffu, give.y, 1)));
+    }
+    const float2 give = lz ? s[0] : s[1], own = lz ? s[1] : s[0];
+    const float2 val = __fadd2_rn(own, make_float2(__shfl_xor_sync(0xffffffffu, give.x, 2),
+                                                   __shfl_xor_sync(0xffffffffu, give.y, 2)));
+    const int u = u0 + 2 * ly + su, v = v0 + 4 * lz + sv;
+    if (u < g.ncols && v < n) hbuf[((size_t)blockIdx.z * g.ncols + u) * g.ldh + v] = val;
+  }
 }
 
 __global__ void __launch_bounds__(kWarps * 32)
@@ -865,9 +939,7 @@ static int launch_front(const SliceGeom& g, const float2* grid, const cjx_image_
       const bool spline = (g.flags & CJX_GRID_SPLINE) != 0;
       const int64_t map = tn.tile;
 #define CJX_GSM(S, M)                                                                                   \
-  if (spline && pairs)                                                                                  \
-    k_gather_slice<S, SplinePairLayout, M><<<gg, 256, 0, stream>>>(grid, params, order, hb, g, k0);   \
-  else if (spline && bricked)                                                                           \
+  if (spline && bricked)                                                                           \
     k_gather_slice<S, SplineBrickLayout, M><<<gg, 256, 0, stream>>>(grid, params, order, hb, g, k0);  \
   else if (spline)                                                                                      \
     k_gather_slice<S, SplineLinearLayout, M><<<gg, 256, 0, stream>>>(grid, params, order, hb, g, k0); \
@@ -885,7 +957,10 @@ static int launch_front(const SliceGeom& g, const float2* grid, const cjx_image_
   } else {              \
     CJX_GSM(S, 0)       \
   }
-      if (ilp == 4) {
+      if (spline && pairs) {
+        const dim3 gt((g.ncols + 15) / 16, (g.n + 16 * kSplineSteps - 1) / (16 * kSplineSteps), cnt);
+        k_gather_spline_team<<<gt, 256, 0, stream>>>(reinterpret_cast<const float4*>(grid), params, order, hb, g, k0);
+      } else if (ilp == 4) {
         CJX_GS(4)
       } else if (ilp == 2) {
         CJX_GS(2)
