@@ -101,15 +101,21 @@ __device__ __forceinline__ void gather_colifft_body(const float2* __restrict__ g
       r22 = (float)Rm[8];
     }
     float2* col = tile + du * stride;
+    // every lane samples (columns past the edge repeat column 0, rows past N low frequencies); only the stores
+    // are guarded.  The row index and its signed frequency are carried in floating point (exact): with the
+    // floor by addition (floor_index) and the one-permute Morton index, 2.90 -> 2.83 ms per 2048 images 320^2.
+    bool act[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) act[s] = true;
+    float row = (float)dv;
 #pragma unroll 1
-    for (int p0 = 0; p0 < R; p0 += S) {
+    for (int p0 = 0; p0 < R; p0 += S, row += 32.0f * S) {
       float ox[S], oy[S], oz[S];
-      bool act[S];
       float2 val[S];
 #pragma unroll
       for (int s = 0; s < S; ++s) {
-        act[s] = col_ok && (p0 + s) < R;
-        const float vy = (float)fft_index(act[s] ? 32 * (p0 + s) + dv : 0, n);
+        const float v = row + 32.0f * s;
+        const float vy = v < (float)(n - n / 2) ? v : v - (float)n;
         ox[s] = fmaf(r01, vy, bx);
         oy[s] = fmaf(r11, vy, by);
         oz[s] = fmaf(r21, vy, bz);
@@ -123,7 +129,7 @@ __device__ __forceinline__ void gather_colifft_body(const float2* __restrict__ g
       gather_samples<S>(grid, n, L, ox, oy, oz, act, wrap, g.fill, val);
 #pragma unroll
       for (int s = 0; s < S; ++s)
-        if (act[s]) col[pad16(32 * (p0 + s) + dv)] = val[s];
+        if (col_ok && (p0 + s) < R) col[pad16(32 * (p0 + s) + dv)] = val[s];
     }
   }
   __syncthreads();
