@@ -413,8 +413,9 @@ class TemplateSharingSearch:
             m = e - s
             nat.gemm(y16[s:e], self.s16, num, m=m, n=T, k=2 * kp, flags=nat.CJX_GEMM_F16)
             nat.gemm(z16[s:e], self.p16, den, m=m, n=T, k=kp, flags=nat.CJX_GEMM_F16)
-            nat.ncc_argmax(num, den, m, T, oo[s:e], yinv[s:e], zinv[s:e], best_score[s:e], best[s:e],
-                           scores=None if scores is None else scores[s:e])
+            if top is None or scores is not None:  # with re-ranking the FP16 best itself is not returned
+                nat.ncc_argmax(num, den, m, T, oo[s:e], yinv[s:e], zinv[s:e], best_score[s:e], best[s:e],
+                               scores=None if scores is None else scores[s:e])
             if top is not None:
                 nat.ncc_topk(num, den, m, T, oo[s:e], yinv[s:e], zinv[s:e], rerank_top, top[s:e])
         if top is None:
