@@ -59,7 +59,8 @@ __device__ __forceinline__ int fft_index(int i, int n) { return (i < n - n / 2) 
 // from sample win_src(m) of the unshifted length-n_src signal, or is zero
 // padding when win_src returns -1.
 __device__ __forceinline__ int win_src(int m, int n_src, int n_dst, int pad_left) {
-  const int mm = (m + n_dst / 2) % n_dst;  // position in the centred destination
+  int mm = m + n_dst / 2;  // position in the centred destination (m < n_dst: one wrap at most)
+  if (mm >= n_dst) mm -= n_dst;
   int s;
   if (n_dst <= n_src) {
     s = mm + (n_src / 2 - n_dst / 2);
@@ -67,7 +68,8 @@ __device__ __forceinline__ int win_src(int m, int n_src, int n_dst, int pad_left
     s = mm - pad_left;
     if (s < 0 || s >= n_src) return -1;
   }
-  return (s - n_src / 2 + n_src) % n_src;
+  s -= n_src / 2;
+  return s < 0 ? s + n_src : s;
 }
 
 // floor(o) of a grid offset: adding 1.5 2^23 with rounding towards -inf leaves
@@ -126,7 +128,7 @@ __device__ __forceinline__ AxisNodes axis_nodes(float off, int n, bool wrap_nega
 
 // The weighted sum of a sample's 8 corners v[4 dz + 2 dy + dx], w = the lower
 // and upper weights along x, y, z: one running sum per z corner, then their
-// sum (the order in which two lanes share a sample, sample_pairs_team2).
+// sum.
 __device__ __forceinline__ float2 combine_corners(const float2* v, const float* w) {
   float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll

@@ -2,11 +2,11 @@
 //
 // One warp transforms one length-n complex sequence held in shared memory,
 // out of place between two buffers (Stockham autosort, natural order in and
-// out).  Radices 8, 4, 2, 3, 5 have hand-written butterflies, radix 7 uses
-// the twiddle table; a length with any other prime factor falls back to a
-// direct O(n^2) DFT.  Twiddles exp(-2 pi i m / n) are computed per launch in
-// double precision and stored as float2 in shared memory.  The register FFTs
-// (n = 32 R) copy theirs from tables the compiler evaluates.
+// out).  Radices 2 to 10 and 12 have butterflies in registers; a prime factor
+// above 7 takes one stage of its own (prime_stage).  Twiddles
+// exp(-2 pi i m / n) are computed per launch in double precision and stored as
+// float2 in shared memory.  The register FFTs (n = 32 R) copy theirs from
+// tables the compiler evaluates.
 //
 // Sign convention: DIR = -1 is the forward transform (numpy.fft.fft),
 // DIR = +1 the unnormalised inverse (n * numpy.fft.ifft).
@@ -18,26 +18,67 @@
 
 namespace cjx {
 
-constexpr int kMaxStages = 16;
+constexpr int kMaxStages = 12;  // lengths up to 1026 have at most 10 prime factors
 
 struct FftPlan {
   int n;
-  int nstages;  // 0 => direct DFT
+  int nstages;  // 0 only for n = 1
   int radix[kMaxStages];
 };
 
+// Instructions that one warp issues for a stage of radix r over n points: the
+// rounds of 32 butterflies, each with its index arithmetic, r loads, twiddles
+// and stores (about 10 per point) and the butterfly's additions and products.
+__host__ inline int fft_stage_cost(int r, int n) {
+  static const int butterfly[13] = {0, 0, 4, 14, 16, 36, 42, 70, 56, 92, 100, 0, 110};
+  return ((n / r + 31) / 32) * (20 + 10 * r + butterfly[r]);
+}
+
+// The cheapest product of radices <= rmax that gives m; best holds the cheapest so far.
+__host__ inline void fft_plan_search(int m, int rmax, int n, int cost, FftPlan& cur, FftPlan& best, int& best_cost) {
+  static const int radices[] = {12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+  if (cost >= best_cost) return;
+  if (m == 1) {
+    best = cur;
+    best_cost = cost;
+    return;
+  }
+  for (int r : radices) {
+    if (r > rmax || m % r) continue;
+    cur.radix[cur.nstages++] = r;
+    fft_plan_search(m / r, r, n, cost + fft_stage_cost(r, n), cur, best, best_cost);
+    --cur.nstages;
+  }
+}
+
+// Bound by instructions.  512 images 180^2 from N = 360 (5 x 6 x 12 and
+// 5 x 6 x 6 instead of 8 x 5 x 3 x 3 and 4 x 5 x 3 x 3; a multiplication in
+// place of the two divisions per butterfly; a quadrant of twiddles evaluated
+// instead of all; image constants once per CTA; held to 64 registers for 4
+// CTAs per SM): the three resize passes 321 + 252 + 194 us before, 206 + 157 +
+// 149 us now.
+// Prime factors above 7 first, then the odd radices, then the even ones in
+// ascending order: a stage stores at stride (product of the earlier radices)
+// x its own radix, so an odd first radix keeps the first stores free of bank
+// conflicts and a later even one starts from runs of consecutive entries.
 __host__ inline FftPlan make_fft_plan(int n) {
   FftPlan p{};
   p.n = n;
-  int m = n, s = 0;
-  const int radices[] = {8, 4, 2, 3, 5, 7};
-  for (int r : radices) {
-    while (m % r == 0 && s < kMaxStages) {
-      p.radix[s++] = r;
-      m /= r;
+  int m = n;
+  for (int f : {2, 3, 5, 7})
+    while (m % f == 0) m /= f;
+  const int smooth = n / m;
+  for (int f = 11; m > 1; f += 2)
+    while (m % f == 0) {
+      p.radix[p.nstages++] = f;
+      m /= f;
     }
-  }
-  p.nstages = (m == 1) ? s : 0;
+  FftPlan cur{}, best{};
+  int best_cost = 1 << 30;
+  fft_plan_search(smooth, 12, n, 0, cur, best, best_cost);
+  for (int odd = 1; odd >= 0; --odd)
+    for (int s = best.nstages - 1; s >= 0; --s)
+      if ((best.radix[s] & 1) == odd) p.radix[p.nstages++] = best.radix[s];
   return p;
 }
 
@@ -61,11 +102,20 @@ __device__ __forceinline__ float2 twiddle(const float2* tw, int m) {
 }
 
 // Fill tw[m] = exp(-2 pi i m / n), m in [0, n), cooperatively by the block.
+// One quadrant (or half) is evaluated and turned into the others, which gives
+// the same bits: sincospi reduces its argument by quadrants exactly.
 __device__ inline void build_twiddles(float2* tw, int n) {
-  for (int m = threadIdx.x; m < n; m += blockDim.x) {
+  const int parts = (n % 4 == 0) ? 4 : (n % 2 == 0) ? 2 : 1, len = n / parts;
+  for (int m = threadIdx.x; m < len; m += blockDim.x) {
     double s, c;
     sincospi(-2.0 * (double)m / (double)n, &s, &c);
-    tw[m] = make_float2((float)c, (float)s);
+    const float2 w = make_float2((float)c, (float)s);
+    tw[m] = w;
+    if (parts > 1) tw[m + n / 2] = make_float2(-w.x, -w.y);
+    if (parts == 4) {  // times -i, times +i
+      tw[m + len] = make_float2(w.y, -w.x);
+      tw[m + 3 * len] = make_float2(-w.y, w.x);
+    }
   }
 }
 
@@ -139,88 +189,6 @@ __device__ __forceinline__ void dft8(float2* v) {
   v[3] = cadd(e3, o3);
   v[7] = csub(e3, o3);
 }
-
-// Generic radix-R DFT with twiddles exp(DIR 2 pi i r q / R) = tw[(r q n / R) mod n].
-template <int R, int DIR>
-__device__ __forceinline__ void dft_generic(float2* v, const float2* tw, int n) {
-  float2 out[R];
-  const int step = n / R;
-#pragma unroll
-  for (int q = 0; q < R; ++q) {
-    float2 acc = v[0];
-#pragma unroll
-    for (int r = 1; r < R; ++r) acc = cadd(acc, cmul(v[r], twiddle<DIR>(tw, ((r * q) % R) * step)));
-    out[q] = acc;
-  }
-#pragma unroll
-  for (int q = 0; q < R; ++q) v[q] = out[q];
-}
-
-template <int R, int DIR>
-__device__ __forceinline__ void stockham_stage(const float2* __restrict__ in, float2* __restrict__ out,
-                                               int n, int Ns, const float2* tw, int lane) {
-  const int nb = n / R;
-  const int tstep = n / (Ns * R);
-  for (int j = lane; j < nb; j += 32) {
-    const int k = j % Ns;
-    float2 v[R];
-#pragma unroll
-    for (int q = 0; q < R; ++q) v[q] = in[j + q * nb];
-    if (Ns > 1) {
-#pragma unroll
-      for (int q = 1; q < R; ++q) v[q] = cmul(v[q], twiddle<DIR>(tw, (q * k * tstep) % n));
-    }
-    if constexpr (R == 2) dft2<DIR>(v);
-    else if constexpr (R == 3) dft3<DIR>(v);
-    else if constexpr (R == 4) dft4<DIR>(v[0], v[1], v[2], v[3]);
-    else if constexpr (R == 5) dft5<DIR>(v);
-    else if constexpr (R == 8) dft8<DIR>(v);
-    else dft_generic<R, DIR>(v, tw, n);
-    const int base = (j / Ns) * Ns * R + k;
-#pragma unroll
-    for (int q = 0; q < R; ++q) out[base + q * Ns] = v[q];
-  }
-}
-
-// Transform buffer `a` (length plan.n) with scratch `b`; returns the buffer
-// holding the result (a or b).  Executed by one full warp; ends with __syncwarp.
-template <int DIR>
-__device__ float2* warp_fft(float2* a, float2* b, const FftPlan& plan, const float2* tw, int lane) {
-  const int n = plan.n;
-  if (plan.nstages == 0) {
-    for (int k = lane; k < n; k += 32) {
-      float2 acc = make_float2(0.f, 0.f);
-      int m = 0;
-      for (int j = 0; j < n; ++j) {
-        acc = cadd(acc, cmul(a[j], twiddle<DIR>(tw, m)));
-        m += k;
-        if (m >= n) m -= n;
-      }
-      b[k] = acc;
-    }
-    __syncwarp();
-    return b;
-  }
-  int Ns = 1;
-  for (int s = 0; s < plan.nstages; ++s) {
-    const int R = plan.radix[s];
-    switch (R) {
-      case 8: stockham_stage<8, DIR>(a, b, n, Ns, tw, lane); break;
-      case 4: stockham_stage<4, DIR>(a, b, n, Ns, tw, lane); break;
-      case 2: stockham_stage<2, DIR>(a, b, n, Ns, tw, lane); break;
-      case 3: stockham_stage<3, DIR>(a, b, n, Ns, tw, lane); break;
-      case 5: stockham_stage<5, DIR>(a, b, n, Ns, tw, lane); break;
-      default: stockham_stage<7, DIR>(a, b, n, Ns, tw, lane); break;
-    }
-    __syncwarp();
-    float2* t = a;
-    a = b;
-    b = t;
-    Ns *= R;
-  }
-  return a;
-}
-
 
 // ===========================================================================
 // Register FFT for n = 32 R (R in {1, 2, 3, 4, 5, 6, 8, 10, 12, 16}).
@@ -381,6 +349,30 @@ struct RegDft<5, DIR> {
   __device__ __forceinline__ static void run(float2* v) { dft5<DIR>(v); }
 };
 template <int DIR>
+struct RegDft<7, DIR> {  // pairs (r, 7 - r): real factors, X[q] and X[7 - q] from the same products
+  __device__ __forceinline__ static void run(float2* v) {
+    constexpr float c[4] = {1.0f, (float)ct::cos2pi(1, 7), (float)ct::cos2pi(2, 7), (float)ct::cos2pi(3, 7)};
+    constexpr float d[4] = {0.0f, (float)ct::sin2pi(1, 7), (float)ct::sin2pi(2, 7), (float)ct::sin2pi(3, 7)};
+    const float2 x0 = v[0];
+    const float2 s1 = cadd(v[1], v[6]), s2 = cadd(v[2], v[5]), s3 = cadd(v[3], v[4]);
+    const float2 d1 = csub(v[1], v[6]), d2 = csub(v[2], v[5]), d3 = csub(v[3], v[4]);
+    v[0] = cadd(cadd(x0, s1), cadd(s2, s3));
+    pair(v[1], v[6], x0, s1, s2, s3, c[1], c[2], c[3], d1, d2, d3, d[1], d[2], d[3]);
+    pair(v[2], v[5], x0, s1, s2, s3, c[2], c[3], c[1], d1, d2, d3, d[2], -d[3], -d[1]);
+    pair(v[3], v[4], x0, s1, s2, s3, c[3], c[1], c[2], d1, d2, d3, d[3], -d[1], d[2]);
+  }
+  __device__ __forceinline__ static void pair(float2& up, float2& down, float2 x0, float2 s1, float2 s2, float2 s3,
+                                              float c1, float c2, float c3, float2 d1, float2 d2, float2 d3, float e1,
+                                              float e2, float e3) {
+    const float2 a = make_float2(fmaf(c3, s3.x, fmaf(c2, s2.x, fmaf(c1, s1.x, x0.x))),
+                                 fmaf(c3, s3.y, fmaf(c2, s2.y, fmaf(c1, s1.y, x0.y))));
+    const float2 b = cmul_i<DIR>(make_float2(fmaf(e3, d3.x, fmaf(e2, d2.x, e1 * d1.x)),
+                                             fmaf(e3, d3.y, fmaf(e2, d2.y, e1 * d1.y))));
+    up = cadd(a, b);
+    down = csub(a, b);
+  }
+};
+template <int DIR>
 struct RegDft<8, DIR> {
   __device__ __forceinline__ static void run(float2* v) { dft8<DIR>(v); }
 };
@@ -426,9 +418,157 @@ struct RegDft<6, DIR> : RegDftAB<2, 3, DIR> {};
 template <int DIR>
 struct RegDft<10, DIR> : RegDftAB<2, 5, DIR> {};
 template <int DIR>
+struct RegDft<9, DIR> : RegDftAB<3, 3, DIR> {};
+template <int DIR>
 struct RegDft<12, DIR> : RegDftAB<4, 3, DIR> {};
 template <int DIR>
 struct RegDft<16, DIR> : RegDftAB<4, 4, DIR> {};
+
+// ===========================================================================
+// Shared-memory FFT of any length up to CJX_MAX_SIDE.
+// ===========================================================================
+
+// j / d for j < 1024 and d in [1, 1024] by one multiplication with
+// div_inverse(d): ceil(2^21 / d) d - 2^21 < d, and j d <= 2^20.
+__device__ __forceinline__ unsigned div_inverse(int d) { return ((1u << 21) + (unsigned)d - 1u) / (unsigned)d; }
+__device__ __forceinline__ int div_by(int j, unsigned inverse) { return (int)(((unsigned)j * inverse) >> 21); }
+
+template <int R, int DIR>
+__device__ __forceinline__ void stockham_stage(const float2* __restrict__ in, float2* __restrict__ out,
+                                               int n, int Ns, const float2* tw, int lane) {
+  const int nb = n / R;
+  const int tstep = n / (Ns * R);
+  const unsigned inv = div_inverse(Ns);
+  for (int j = lane; j < nb; j += 32) {
+    const int g = div_by(j, inv), k = j - g * Ns;
+    float2 v[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) v[q] = in[j + q * nb];
+    if (Ns > 1) {  // q k tstep < n
+      const float2* w = tw;
+#pragma unroll
+      for (int q = 1; q < R; ++q) {
+        w += k * tstep;
+        v[q] = cmul(v[q], twiddle<DIR>(w, 0));
+      }
+    }
+    RegDft<R, DIR>::run(v);
+    float2* o = out + g * Ns * R + k;
+#pragma unroll
+    for (int q = 0; q < R; ++q) o[q * Ns] = v[q];
+  }
+}
+
+// Stage of a prime radix p > 7, in two steps.  First every pair of inputs
+// (r, p - r) is replaced by its sum and difference (in overwrites itself);
+// then X[q] and X[p - q] come from the same products,
+//   X[q], X[p - q] = x_0 + sum_r s_r cos(2 pi r q / p) +- i sum_r d_r sin(...),
+// real factors on (p - 1) / 2 pairs: a quarter of the multiplications of the
+// direct sum.  A lane keeps Q outputs, so that each pair read serves all of them.
+template <int Q, int DIR>
+__device__ __forceinline__ void prime_outputs(const float2* __restrict__ in, float2* __restrict__ out, int n, int p,
+                                              int Ns, const float2* tw, int lane) {
+  const int nb = n / p, half = (p - 1) / 2, groups = half / Q + 1;
+  const unsigned inv_nb = div_inverse(nb), inv_ns = div_inverse(Ns);
+  for (int t = lane; t < nb * groups; t += 32) {
+    const int qg = div_by(t, inv_nb), j = t - qg * nb;
+    const float2 x0 = in[j];
+    float2 A[Q], B[Q];
+    int m[Q], step[Q];
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+      A[i] = x0;
+      B[i] = make_float2(0.f, 0.f);
+      m[i] = 0;
+      step[i] = min(Q * qg + i, half) * nb;
+    }
+    const float2* lo = in + j;
+    const float2* hi = in + j + n;
+    for (int r = 1; r <= half; ++r) {
+      lo += nb;
+      hi -= nb;
+      const float2 s = *lo, d = *hi;
+#pragma unroll
+      for (int i = 0; i < Q; ++i) {
+        m[i] += step[i];
+        if (m[i] >= n) m[i] -= n;
+        const float2 w = tw[m[i]];
+        A[i].x = fmaf(s.x, w.x, A[i].x);
+        A[i].y = fmaf(s.y, w.x, A[i].y);
+        B[i].x = fmaf(d.x, w.y, B[i].x);
+        B[i].y = fmaf(d.y, w.y, B[i].y);
+      }
+    }
+    const int g = div_by(j, inv_ns);
+    float2* o = out + g * Ns * p + (j - g * Ns);
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+      const int q = Q * qg + i;
+      const float2 b = DIR < 0 ? make_float2(-B[i].y, B[i].x) : make_float2(B[i].y, -B[i].x);
+      if (q <= half) o[q * Ns] = cadd(A[i], b);
+      if (q > 0 && q <= half) o[(p - q) * Ns] = csub(A[i], b);
+    }
+  }
+}
+
+template <int DIR>
+__device__ __noinline__ void prime_stage(float2* __restrict__ in, float2* __restrict__ out, int n, int p, int Ns,
+                                         const float2* tw, int lane) {
+  const int nb = n / p, half = (p - 1) / 2;
+  const int tstep = n / (Ns * p);
+  const unsigned inv_nb = div_inverse(nb), inv_ns = div_inverse(Ns);
+  for (int e = lane; e < nb * half; e += 32) {
+    const int r = 1 + div_by(e, inv_nb), j = e - (r - 1) * nb;
+    const int k = j - div_by(j, inv_ns) * Ns;
+    float2 a = in[j + r * nb], b = in[j + (p - r) * nb];
+    if (Ns > 1) {
+      a = cmul(a, twiddle<DIR>(tw, r * k * tstep));
+      b = cmul(b, twiddle<DIR>(tw, (p - r) * k * tstep));
+    }
+    in[j + r * nb] = cadd(a, b);
+    in[j + (p - r) * nb] = csub(a, b);
+  }
+  __syncwarp();
+  if (nb * (half / 4 + 1) >= 20)  // enough lanes busy with four outputs each
+    prime_outputs<4, DIR>(in, out, n, p, Ns, tw, lane);
+  else
+    prime_outputs<1, DIR>(in, out, n, p, Ns, tw, lane);
+}
+
+// Transform buffer `a` (length plan.n) with scratch `b`; returns the buffer
+// holding the result (a or b).  Executed by one full warp; ends with __syncwarp.
+template <int DIR>
+__device__ float2* warp_fft(float2* a, float2* b, const FftPlan& plan, const float2* tw, int lane) {
+  const int n = plan.n;
+  if (plan.nstages == 0) {  // n = 1
+    if (lane == 0) b[0] = a[0];
+    __syncwarp();
+    return b;
+  }
+  int Ns = 1;
+  for (int s = 0; s < plan.nstages; ++s) {
+    const int R = plan.radix[s];
+    switch (R) {
+      case 2: stockham_stage<2, DIR>(a, b, n, Ns, tw, lane); break;
+      case 3: stockham_stage<3, DIR>(a, b, n, Ns, tw, lane); break;
+      case 4: stockham_stage<4, DIR>(a, b, n, Ns, tw, lane); break;
+      case 5: stockham_stage<5, DIR>(a, b, n, Ns, tw, lane); break;
+      case 6: stockham_stage<6, DIR>(a, b, n, Ns, tw, lane); break;
+      case 7: stockham_stage<7, DIR>(a, b, n, Ns, tw, lane); break;
+      case 8: stockham_stage<8, DIR>(a, b, n, Ns, tw, lane); break;
+      case 9: stockham_stage<9, DIR>(a, b, n, Ns, tw, lane); break;
+      case 10: stockham_stage<10, DIR>(a, b, n, Ns, tw, lane); break;
+      case 12: stockham_stage<12, DIR>(a, b, n, Ns, tw, lane); break;
+      default: prime_stage<DIR>(a, b, n, R, Ns, tw, lane); break;
+    }
+    __syncwarp();
+    float2* t = a;
+    a = b;
+    b = t;
+    Ns *= R;
+  }
+  return a;
+}
 
 // Per-lane twiddles of the 5 cross-lane DIT stages (forward sign):
 // stage s (span h = 2^s) uses exp(-2 pi i (l mod h) / (2h)) =

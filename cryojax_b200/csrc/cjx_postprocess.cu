@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kWarps * 32)
   float2* oa = out + ((size_t)blockIdx.y * py + ra) * pxh;
   for (int k = lane; k < pxh; k += 32) {
     const float2 Zk = Z[k];
-    const float2 Zm = Z[(px - k) % px];
+    const float2 Zm = Z[k == 0 ? 0 : px - k];
     oa[k] = make_float2(0.5f * (Zk.x + Zm.x), 0.5f * (Zk.y - Zm.y));
     if (has_b) oa[pxh + k] = make_float2(0.5f * (Zk.y + Zm.y), -0.5f * (Zk.x - Zm.x));
   }

@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(256, 4)
   }
 }
 
-__global__ void __launch_bounds__(kWarps * 32)
+__global__ void __launch_bounds__(kWarps * 32, 4)
     k_colifft_window(const float2* __restrict__ hbuf, float2* __restrict__ t1, SliceGeom g) {
   extern __shared__ float2 smem[];
   const int n = g.n, h = n / 2;
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kWarps * 32)
 // ---------------------------------------------------------------------------
 // Pass B
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kWarps * 32)
+__global__ void __launch_bounds__(kWarps * 32, 4)
     k_rows_c2r_r2c(const float2* __restrict__ t1, float2* __restrict__ t2, SliceGeom g) {
   extern __shared__ float2 smem[];
   const int n = g.n, px = g.px;
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(kWarps * 32)
   float2* outA = t2 + ((size_t)blockIdx.y * g.py + ra) * g.ld2;
   for (int k = lane; k < g.pxh; k += 32) {
     const float2 Wk = W[k];
-    const float2 Wm = W[(px - k) % px];
+    const float2 Wm = W[k == 0 ? 0 : px - k];
     outA[k] = make_float2(0.5f * (Wk.x + Wm.x), 0.5f * (Wk.y - Wm.y));
     if (has_b) outA[g.ld2 + k] = make_float2(0.5f * (Wk.y + Wm.y), -0.5f * (Wk.x - Wm.x));
   }
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(kWarps * 32)
 // ---------------------------------------------------------------------------
 // Pass C
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kWarps * 32)
+__global__ void __launch_bounds__(kWarps * 32, 4)
     k_colfft_epilogue(const float2* __restrict__ t2, const cjx_image_params* __restrict__ params,
                       const int32_t* __restrict__ order, float2* __restrict__ out, SliceGeom g, int64_t k0,
                       float norm) {
@@ -362,6 +362,7 @@ __global__ void __launch_bounds__(kWarps * 32)
   const int stride = 2 * py + 2;
   float2* tw = smem;
   float2* bufs = smem + py;
+  ImageConsts& sc = *reinterpret_cast<ImageConsts*>(bufs + kWarps * stride);
   build_twiddles(tw, py);
 
   const int j0 = blockIdx.x * kWarps;
@@ -373,8 +374,10 @@ __global__ void __launch_bounds__(kWarps * 32)
   }
   const int64_t k = k0 + blockIdx.y;
   const int64_t img = order ? (int64_t)order[k] : k;
-  const ImageConsts c = load_image_consts(params + img, norm, g.py, g.px);
+  // once per CTA: its double divisions and sincos in every thread took as long as the transforms
+  if (threadIdx.x == 0) sc = load_image_consts(params + img, norm, g.py, g.px);
   __syncthreads();
+  const ImageConsts& c = sc;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp < ncols) {
@@ -529,7 +532,7 @@ __device__ __forceinline__ void rows_pair_reg(float2 (&z)[RN], bool has_b, float
   __syncwarp();
   for (int k = lane; k <= px / 2; k += 32) {
     const float2 Wk = buf[stage_r(RP, k)];
-    const float2 Wm = buf[stage_r(RP, (px - k) % px)];
+    const float2 Wm = buf[stage_r(RP, k == 0 ? 0 : px - k)];
     outA[k] = make_float2(0.5f * (Wk.x + Wm.x), 0.5f * (Wk.y - Wm.y));
     if (has_b) outA[ld2 + k] = make_float2(0.5f * (Wk.y + Wm.y), -0.5f * (Wk.x - Wm.x));
   }
@@ -749,7 +752,9 @@ static size_t smem_b(const SliceGeom& g) {
   const int L = std::max(g.n, g.px);
   return sizeof(float2) * (size_t)(g.n + g.px + kWarps * (2 * L + 2));
 }
-static size_t smem_c(const SliceGeom& g) { return sizeof(float2) * (size_t)(g.py + kWarps * (2 * g.py + 2)); }
+static size_t smem_c(const SliceGeom& g) {
+  return sizeof(float2) * (size_t)(g.py + kWarps * (2 * g.py + 2)) + sizeof(ImageConsts);
+}
 
 // Process-wide tuning knobs (cjx_tuning_set / cjx_tuning_get).
 static std::atomic<int64_t> g_gather_ilp{2};
