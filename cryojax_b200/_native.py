@@ -343,6 +343,14 @@ _SIGNATURES = {
         ctypes.c_int,
         [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p],
     ),
+    "cjx_pack_image_params": (
+        ctypes.c_int,
+        [ctypes.c_int64, ctypes.c_uint32, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]),
+    "cjx_orientation_order": (
+        ctypes.c_int, [ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int, ctypes.c_void_p]),
+    "cjx_quaternion_grad": (
+        ctypes.c_int,
+        [ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]),
     "cjx_profile_enable": (ctypes.c_int, [ctypes.c_int]),
     "cjx_profile_read": (
         ctypes.c_int,
@@ -987,6 +995,76 @@ def profile_read(max_kernels: int = 32) -> dict:
     for i in range(n.value):
         name = names.raw[32 * i: 32 * (i + 1)].split(b"\0", 1)[0].decode()
         out[name] = (int(counts[i]), float(ms[i]))
+    return out
+
+
+CJX_PACK_NORMALISE, CJX_PACK_THEORY, CJX_PACK_ENVELOPE = 1, 2, 4
+
+
+def _address(a) -> int:
+    return a.__array_interface__["data"][0]
+
+
+def _rows(a, n: int, width: int):
+    """(array, stride in doubles) of float64 rows [width] shared by all images, or [m, ..., width] with one per image."""
+    if a.ndim > 1:
+        a = a.reshape(-1, width)
+        if a.shape[0] == n:
+            a = np.ascontiguousarray(a)
+            return a, width
+        a = np.ascontiguousarray(np.broadcast_to(a, (n, width)))  # one row for all, or an error
+        return a, width
+    return np.ascontiguousarray(a), 0
+
+
+def _column(a, n: int):
+    """(array, stride in doubles) of a float64 scalar shared by all images, or of one value per image."""
+    if a.ndim == 0:
+        return a, 0
+    a = a.reshape(a.shape[0])
+    if a.shape[0] != n:
+        if a.shape[0] != 1:
+            np.broadcast_to(a, (n,))  # raises
+        return a, 0
+    if a.strides[0] % 8:
+        a = np.ascontiguousarray(a)
+    return a, a.strides[0] // 8
+
+
+def pack_image_params(n: int, quaternion, offset, columns, *, normalise: bool) -> np.ndarray:
+    """cjx_pack_image_params: float64 [n, 32] records.  ``columns``: float64 arrays (0-d or one value per image) of
+    pixel size, kilovolts and scale; then, of a transfer theory, defocus, astigmatism, angle, aberration, contrast
+    ratio, phase shift; then, of an envelope, amplitude and b-factor."""
+    width = offset.shape[-1]
+    kept = [_rows(quaternion, n, 4), _rows(offset, n, width)] + [_column(c, n) for c in columns]
+    flags = (CJX_PACK_NORMALISE if normalise else 0) | (CJX_PACK_THEORY if len(columns) > 3 else 0) | (
+        CJX_PACK_ENVELOPE if len(columns) > 9 else 0)
+    sources = (ctypes.c_void_p * 13)(*[_address(a) for a, _ in kept])
+    strides = (ctypes.c_int64 * 13)(*[s for _, s in kept])
+    out = np.empty((n, PARAMS_DOUBLES), np.float64)
+    _check(load_library().cjx_pack_image_params(n, flags, width, sources, strides, _address(out)))
+    return out
+
+
+def orientation_order(rotations, bits: int) -> np.ndarray:
+    """cjx_orientation_order of float64 [n, 3, 3] rotations (or a view of them in longer rows): int32 [n]."""
+    R = rotations
+    if R.strides[-2:] != (24, 8) or R.strides[0] % 8:
+        R = np.ascontiguousarray(R)
+    order = np.empty(R.shape[0], np.int32)
+    if R.shape[0]:
+        _check(load_library().cjx_orientation_order(R.shape[0], _address(R), R.strides[0] // 8, int(bits),
+                                                    _address(order)))
+    return order
+
+
+def quaternion_grad(wxyz, d_rotation) -> np.ndarray:
+    """cjx_quaternion_grad: float64 [n, 4] from quaternions [n, 4] (or [1, 4]) and dL/dR [n, 3, 2 or 3]."""
+    n, _, columns = d_rotation.shape
+    q, stride = _rows(wxyz, n, 4)
+    g = np.ascontiguousarray(d_rotation)
+    out = np.empty((n, 4), np.float64)
+    _check(load_library().cjx_quaternion_grad(n, _address(q), stride, _address(g), columns, _address(out)))
     return out
 
 

@@ -12,7 +12,8 @@ The device computes dL/dR (rotation matrix columns that span the slice
 plane), dL/d(shift), dL/d(defocus) and the trilinear scatter-add for the
 grid (cjx_slice_ctf_loss_grad).  The last step, from dL/dR to the pose's own
 parameters (quaternion through its normalisation, zyz Euler angles in
-degrees, or an axis-angle vector), is a float64 autograd on the host.
+degrees, or an axis-angle vector), runs on the host in float64: the
+quaternion's in native code (cjx_quaternion_grad), the others' as an autograd.
 Complex gradients are dL/dRe + i dL/dIm (jax.grad returns the conjugate).
 """
 
@@ -104,6 +105,19 @@ def _pose_param_array(pose, n):
     raise TypeError(f"unsupported pose type {type(pose).__name__}")
 
 
+def _pose_gradient(pose, values, d_rot):
+    """dL/d(pose parameters) (n, k) of dL/dR (n, 3, 2 or 3) at the parameter values (n, k)."""
+    from .simulator import QuaternionPose
+
+    if isinstance(pose, QuaternionPose):
+        return nat.quaternion_grad(np.asarray(values, np.float64), d_rot)
+    torch = _torch()
+    p_t = torch.tensor(np.ascontiguousarray(values), dtype=torch.float64, requires_grad=True)
+    R = _pose_rotation_t(pose, p_t)
+    (R[:, :, 0:d_rot.shape[2]] * torch.as_tensor(d_rot)).sum().backward()
+    return p_t.grad.numpy().copy()
+
+
 def observed_to_fourier(observed):
     """cryoJAX rfftn of real-space images (ifftshift, then rfft2): complex64 [n, Py, Px//2+1]."""
     torch = _torch()
@@ -137,6 +151,7 @@ def squared_residual_and_grad(model, observed, *, grid_grad: bool = True, observ
         raise NotImplementedError("the loss gradient needs padded_shape == shape")
     vol = model.volume_parametrization.get_representation()
     integ = model.volume_integrator
+    obs_f = observed if observed_is_fourier else observed_to_fourier(observed)  # runs while the host packs
     params = model.image_params()
     n = params.shape[0]
     ewald = not integ.is_projection_approximation  # EwaldSphereExtraction: R's third column enters too
@@ -159,7 +174,6 @@ def squared_residual_and_grad(model, observed, *, grid_grad: bool = True, observ
         flags |= layout
     py, px = cfg.padded_shape
     desc = nat.make_desc(vol.shape[0], py, px, flags, integ.fill_value)
-    obs_f = observed if observed_is_fourier else observed_to_fourier(observed)
     if tuple(obs_f.shape) != (n, py, px // 2 + 1):
         raise ValueError(f"observed has shape {tuple(obs_f.shape)}, expected {(n, py, px // 2 + 1)} in Fourier space")
     pd = torch.as_tensor(params, device=dev)
@@ -174,14 +188,12 @@ def squared_residual_and_grad(model, observed, *, grid_grad: bool = True, observ
     d_rot = g[:, nat.G_ROT:nat.G_ROT + 6].reshape(n, 3, 2)
     if ewald:  # the third column's entries follow the first two columns'
         d_rot = np.concatenate([d_rot, g[:, nat.G_ROT + 6:nat.G_ROT + 9, None]], axis=2)
-    # chain dL/dR -> pose parameters (float64 autograd on the host)
+    # chain dL/dR -> pose parameters (float64, on the host)
     pvals, pname = _pose_param_array(model.pose, n)
-    p_t = torch.tensor(np.ascontiguousarray(pvals), dtype=torch.float64, requires_grad=True)
-    R = _pose_rotation_t(model.pose, p_t)
-    (R[:, :, 0:d_rot.shape[2]] * torch.as_tensor(d_rot)).sum().backward()
+    p_grad = _pose_gradient(model.pose, pvals, d_rot)
     out = {
         "loss": g[:, nat.G_LOSS].copy(),
-        pname: p_t.grad.numpy().copy(),
+        pname: p_grad,
         "d_offset": g[:, nat.G_TX:nat.G_TY + 1].copy(),
         "d_defocus": g[:, nat.G_DF].copy(),
         "d_rotation": d_rot,

@@ -66,15 +66,8 @@ def _batch_size(*xs) -> int | None:
     return n
 
 
-def _per_image(x, n):
-    a = _arr(x)
-    if a.ndim == 0:
-        return np.full(n, float(a))
-    return np.broadcast_to(a.reshape(a.shape[0]), (n,)).astype(np.float64)
-
-
 def _require_positive(name, x):
-    if np.any(_arr(x) <= 0):
+    if (_arr(x) <= 0).any():
         raise ValueError(f"`{name}` must be positive")
 
 
@@ -216,7 +209,7 @@ class AstigmaticCTF:
 
     def __init__(self, defocus_in_angstroms=10000.0, astigmatism_in_angstroms=0.0, astigmatism_angle=0.0,
                  spherical_aberration_in_mm=2.7):
-        if np.any(_arr(spherical_aberration_in_mm) < 0):
+        if (_arr(spherical_aberration_in_mm) < 0).any():
             raise ValueError("`spherical_aberration_in_mm` must be non-negative")
         self.defocus_in_angstroms = _arr(defocus_in_angstroms)
         self.astigmatism_in_angstroms = _arr(astigmatism_in_angstroms)
@@ -261,7 +254,7 @@ class ContrastTransferTheory:
     def __init__(self, ctf: AstigmaticCTF, envelope: FourierGaussian | Constant | None = None,
                  amplitude_contrast_ratio=0.1, phase_shift=0.0):
         ac = _arr(amplitude_contrast_ratio)
-        if np.any(ac < 0) or np.any(ac > 1):
+        if ((ac < 0) | (ac > 1)).any():
             raise ValueError("`amplitude_contrast_ratio` must be in [0, 1]")
         if envelope is not None and not isinstance(envelope, (FourierGaussian, Constant)):
             raise NotImplementedError("only FourierGaussian and Constant envelopes run on the device")
@@ -566,74 +559,28 @@ class GaussianMixtureRenderFn:
 def pack_image_params(pose: AbstractPose, image_config: BasicImageConfig,
                       transfer_theory: ContrastTransferTheory | None = None, scale=1.0, n: int | None = None):
     """Build the float64 [n, 32] cjx_image_params records for a batch."""
-    q = pose.quaternion()
-    ctf = transfer_theory.ctf if transfer_theory is not None else None
-    cands = [q if q.ndim > 1 else None, pose.offset_in_angstroms if pose.offset_in_angstroms.ndim > 1 else None,
-             image_config.pixel_size, image_config.voltage_in_kilovolts, scale]
+    normalise = type(pose) is QuaternionPose  # q / |q| of its own values is left to the native packing
+    q = _arr(pose.wxyz if normalise else pose.quaternion())
+    if q.ndim > 2 and q.size > 4:
+        raise ValueError(f"expected one quaternion, or one per image, got shape {q.shape}")
+    off = _arr(pose.offset_in_angstroms)
+    columns = [image_config.pixel_size, image_config.voltage_in_kilovolts, scale]
     if transfer_theory is not None:
-        cands += [ctf.defocus_in_angstroms, ctf.astigmatism_in_angstroms, ctf.astigmatism_angle,
-                  ctf.spherical_aberration_in_mm, transfer_theory.amplitude_contrast_ratio,
-                  transfer_theory.phase_shift]
+        ctf = transfer_theory.ctf
+        columns += [ctf.defocus_in_angstroms, ctf.astigmatism_in_angstroms, ctf.astigmatism_angle,
+                    ctf.spherical_aberration_in_mm, transfer_theory.amplitude_contrast_ratio,
+                    transfer_theory.phase_shift]
         if transfer_theory.envelope is not None:
-            cands += list(_envelope_amp_b(transfer_theory.envelope))
+            columns += _envelope_amp_b(transfer_theory.envelope)
+    columns = [_arr(c) for c in columns]
     if n is None:
-        n = _batch_size(*cands) or 1
-    p = nat.empty_params(n)
-    R = rot.quat_to_matrix(q)
-    p[:, 0:9] = np.broadcast_to(R.reshape(-1, 9) if R.ndim == 3 else R.reshape(1, 9), (n, 9))
-    off = pose.offset_in_angstroms
-    off = off.reshape(-1, off.shape[-1]) if off.ndim > 1 else off[None]
-    off = np.broadcast_to(off, (n, off.shape[-1]))
-    p[:, nat.P_SHIFT_X] = off[:, 0]
-    p[:, nat.P_SHIFT_Y] = off[:, 1]
-    px = _per_image(image_config.pixel_size, n)
-    kv = _per_image(image_config.voltage_in_kilovolts, n)
-    p[:, nat.P_PIXEL_SIZE] = px
-    p[:, nat.P_WAVELENGTH] = C.wavelength_from_kilovolts(kv)
-    p[:, nat.P_SCALE] = _per_image(scale, n)
-    if transfer_theory is not None:
-        df = _per_image(ctf.defocus_in_angstroms, n)
-        if off.shape[-1] == 3:
-            df = df + off[:, 2]
-        p[:, nat.P_DEFOCUS] = df
-        p[:, nat.P_ASTIG] = _per_image(ctf.astigmatism_in_angstroms, n)
-        p[:, nat.P_ASTIG_ANGLE] = np.deg2rad(_per_image(ctf.astigmatism_angle, n))
-        p[:, nat.P_CS] = _per_image(ctf.spherical_aberration_in_mm, n) * 1e7
-        ac = _per_image(transfer_theory.amplitude_contrast_ratio, n)
-        p[:, nat.P_PHASE_TOTAL] = np.deg2rad(_per_image(transfer_theory.phase_shift, n)) + np.arctan(
-            ac / np.sqrt(1.0 - ac**2))
-        p[:, nat.P_AC] = ac
-        p[:, nat.P_PHASE_SHIFT] = np.deg2rad(_per_image(transfer_theory.phase_shift, n))
-        if transfer_theory.envelope is not None:
-            amp, b = _envelope_amp_b(transfer_theory.envelope)
-            p[:, nat.P_ENV_AMP] = _per_image(amp, n)
-            p[:, nat.P_ENV_B] = _per_image(b, n)
-    return p
+        n = _batch_size(q if q.ndim > 1 else None, off if off.ndim > 1 else None, *columns) or 1
+    return nat.pack_image_params(n, q, off, columns, normalise=normalise)
 
 
 # ---------------------------------------------------------------------------
 # Processing order
 # ---------------------------------------------------------------------------
-
-
-def _hilbert_index(x, y, order):
-    """Hilbert-curve index of integer points (x, y) in [0, 2^order)^2."""
-    x = x.astype(np.int64).copy()
-    y = y.astype(np.int64).copy()
-    d = np.zeros_like(x)
-    s = 1 << (order - 1)
-    while s > 0:
-        rx = (x & s) > 0
-        ry = (y & s) > 0
-        d += s * s * ((3 * rx) ^ ry)
-        # rotate the quadrant
-        swap = ~ry
-        flip = swap & rx
-        x = np.where(flip, s - 1 - x, x)
-        y = np.where(flip, s - 1 - y, y)
-        x, y = np.where(swap, y, x), np.where(swap, x, y)
-        s >>= 1
-    return d
 
 
 def orientation_order(rotations: np.ndarray, bits: int = 8) -> np.ndarray:
@@ -645,16 +592,7 @@ def orientation_order(rotations: np.ndarray, bits: int = 8) -> np.ndarray:
     ordered along a Hilbert curve.  Consecutive images then touch largely the
     same voxels, which the L2 cache serves once.
     """
-    R = np.asarray(rotations, np.float64).reshape(-1, 3, 3)
-    n = R[:, :, 2].copy()
-    flip = (n[:, 2] < 0) | ((n[:, 2] == 0) & (n[:, 1] < 0))
-    n[flip] *= -1.0
-    k = np.sqrt(2.0 / (1.0 + np.clip(n[:, 2], 0.0, 1.0)))
-    px, py = k * n[:, 0], k * n[:, 1]  # disk of radius sqrt(2)
-    scale = (1 << bits) - 1
-    gx = np.clip(np.round((px / np.sqrt(2.0) + 1.0) * 0.5 * scale), 0, scale)
-    gy = np.clip(np.round((py / np.sqrt(2.0) + 1.0) * 0.5 * scale), 0, scale)
-    return np.argsort(_hilbert_index(gx, gy, bits), kind="stable").astype(np.int32)
+    return nat.orientation_order(np.asarray(rotations, np.float64).reshape(-1, 3, 3), bits)
 
 
 # ---------------------------------------------------------------------------
@@ -863,7 +801,9 @@ class AbstractImageModel:
 
     def _batched_fields(self):
         tt = self.transfer_theory
-        fields = [self.pose.quaternion() if self.pose.quaternion().ndim > 1 else None,
+        pose = self.pose
+        q = pose.wxyz if type(pose) is QuaternionPose else pose.quaternion()
+        fields = [q if q.ndim > 1 else None,
                   self.pose.offset_in_angstroms if self.pose.offset_in_angstroms.ndim > 1 else None,
                   self.image_config.pixel_size, self.image_config.voltage_in_kilovolts]
         if tt is not None:

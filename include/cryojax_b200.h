@@ -656,6 +656,31 @@ CJX_API int cjx_adamw(float* params, const float* grads, float* m, float* v, int
 CJX_API int cjx_topk_candidates(const float* logits, int64_t B, int C, int k, int n_inplane,
                                 int32_t* dirs, int32_t* candidates, void* stream);
 
+/* ---- host-side steps (no device work, no state) ----------------------- */
+#define CJX_PACK_NORMALISE (1u << 0) /* divide the quaternions by their norm first */
+#define CJX_PACK_THEORY (1u << 1)    /* CTF sources given                   */
+#define CJX_PACK_ENVELOPE (1u << 2)  /* envelope sources given (with CJX_PACK_THEORY) */
+/* n_images records from 13 host sources of doubles: quaternion (4 values,
+ * wxyz), offset (offset_dim = 2 or 3 values, Angstrom; the third adds to
+ * the defocus), pixel size, kilovolts, scale; with CJX_PACK_THEORY defocus,
+ * astigmatism (A), its angle (degrees), spherical aberration (mm),
+ * amplitude contrast ratio, phase shift (degrees); with CJX_PACK_ENVELOPE
+ * envelope amplitude and b-factor.  Image i reads source s at
+ * strides[s] * i doubles (0: one value for all images); unused sources may
+ * be NULL.                                                                 */
+CJX_API int cjx_pack_image_params(int64_t n_images, uint32_t flags, int offset_dim, const void* const* sources,
+                                  const int64_t* strides, cjx_image_params* out);
+/* order[n_images]: the images by the Hilbert-curve index (bits per axis) of
+ * their sign-free plane normal R[:, 2] in Lambert's equal-area projection,
+ * ties in input order.  rotations: row-major 3 x 3 doubles, image i at
+ * stride * i doubles.                                                      */
+CJX_API int cjx_orientation_order(int64_t n_images, const double* rotations, int64_t stride, int bits,
+                                  int32_t* order);
+/* dL/d(wxyz) [n][4] of dL/dR [n][3][columns] (R's first 2 or all 3 columns)
+ * for R of q / |q|; image i reads wxyz at quat_stride * i doubles.         */
+CJX_API int cjx_quaternion_grad(int64_t n_images, const double* wxyz, int64_t quat_stride, const double* d_rot,
+                                int columns, double* d_wxyz);
+
 #ifdef __cplusplus
 }
 #endif
