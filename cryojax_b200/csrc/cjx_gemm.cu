@@ -25,59 +25,99 @@ struct GemmEpilogue {
   int flags;
   int M, N;
 
-  __device__ void operator()(int row, int col0, float (&v)[16]) const {
-    if (row >= M) return;
-    const int nv = min(16, N - col0);
-    if (nv <= 0) return;
+  // Bias and ReLU on columns col0.. of one row.
+  __device__ __forceinline__ void finish(int col0, float (&v)[16]) const {
     if (flags & CJX_GEMM_BIAS) {
 #pragma unroll
       for (int i = 0; i < 16; ++i)
-        if (i < nv) v[i] += bias[col0 + i];
+        if (col0 + i < N) v[i] += bias[col0 + i];
     }
     if (flags & CJX_GEMM_RELU) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.f);
     }
-    if (flags & CJX_GEMM_OUT_BF16) {
-      __nv_bfloat16* c = static_cast<__nv_bfloat16*>(C) + (size_t)row * ldc + col0;
-      if (nv == 16 && (reinterpret_cast<uintptr_t>(c) & 15) == 0) {
-        uint32_t w[8];
+  }
+
+  // 32 rows x 32 columns of a warp, lane l holding row l in a and b, through
+  // the warp's staging buffer (32 rows of kPitch floats, conflict-free for the
+  // 16-byte writes and reads), so that a store instruction covers whole
+  // 128-byte lines of a few rows instead of 16 bytes of 32 rows.
+  static constexpr int kPitch = 36;
+  __device__ __forceinline__ void store(float* stage, int row0, int col0, int lane, float (&a)[16],
+                                        float (&b)[16]) const {
+    finish(col0, a);
+    finish(col0 + 16, b);
+    const bool full = col0 + 32 <= N;
+    __syncwarp();  // the previous block's reads
+    if ((flags & CJX_GEMM_OUT_BF16) && full && (ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
+      constexpr int kPitch16 = 20;  // words: 32 BF16 and padding
+      uint32_t* st = reinterpret_cast<uint32_t*>(stage);
+      uint32_t w[16];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-          w[i] = *reinterpret_cast<uint32_t*>(&h);
-        }
-        reinterpret_cast<uint4*>(c)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-        reinterpret_cast<uint4*>(c)[1] = make_uint4(w[4], w[5], w[6], w[7]);
-      } else {
-        for (int i = 0; i < nv; ++i) c[i] = __float2bfloat16_rn(v[i]);
+      for (int i = 0; i < 8; ++i) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(a[2 * i], a[2 * i + 1]);
+        const __nv_bfloat162 g = __floats2bfloat162_rn(b[2 * i], b[2 * i + 1]);
+        w[i] = *reinterpret_cast<const uint32_t*>(&h);
+        w[8 + i] = *reinterpret_cast<const uint32_t*>(&g);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<uint4*>(st + lane * kPitch16 + 4 * i) =
+            make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+      __syncwarp();
+      __nv_bfloat16* c = static_cast<__nv_bfloat16*>(C);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = 8 * i + (lane >> 2), q = lane & 3;
+        const uint4 v = *reinterpret_cast<const uint4*>(st + r * kPitch16 + 4 * q);
+        if (row0 + r < M) *reinterpret_cast<uint4*>(c + (size_t)(row0 + r) * ldc + col0 + 8 * q) = v;
+      }
+      return;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      *reinterpret_cast<float4*>(stage + lane * kPitch + 4 * i) =
+          make_float4(a[4 * i], a[4 * i + 1], a[4 * i + 2], a[4 * i + 3]);
+      *reinterpret_cast<float4*>(stage + lane * kPitch + 16 + 4 * i) =
+          make_float4(b[4 * i], b[4 * i + 1], b[4 * i + 2], b[4 * i + 3]);
+    }
+    __syncwarp();
+    const int rows = min(32, M - row0);
+    if (flags & CJX_GEMM_OUT_BF16) {
+      __nv_bfloat16* c = static_cast<__nv_bfloat16*>(C) + (size_t)row0 * ldc + col0 + lane;
+      if (col0 + lane < N)
+        for (int r = 0; r < rows; ++r) c[(size_t)r * ldc] = __float2bfloat16_rn(stage[r * kPitch + lane]);
+    } else if (flags & CJX_GEMM_ACCUMULATE) {
+      float* c = static_cast<float*>(C) + (size_t)row0 * ldc + col0 + lane;
+      if (col0 + lane < N)
+        for (int r = 0; r < rows; ++r) atomicAdd(c + (size_t)r * ldc, stage[r * kPitch + lane]);
+    } else if (full && (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
+      float* c = static_cast<float*>(C);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = 4 * i + (lane >> 3), q = lane & 7;
+        const float4 v = *reinterpret_cast<const float4*>(stage + r * kPitch + 4 * q);
+        if (row0 + r < M) *reinterpret_cast<float4*>(c + (size_t)(row0 + r) * ldc + col0 + 4 * q) = v;
       }
     } else {
-      float* c = static_cast<float*>(C) + (size_t)row * ldc + col0;
-      if (flags & CJX_GEMM_ACCUMULATE) {
-        for (int i = 0; i < nv; ++i) atomicAdd(c + i, v[i]);
-      } else if (nv == 16 && (reinterpret_cast<uintptr_t>(c) & 15) == 0) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          reinterpret_cast<float4*>(c)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-      } else {
-        for (int i = 0; i < nv; ++i) c[i] = v[i];
-      }
+      float* c = static_cast<float*>(C) + (size_t)row0 * ldc + col0 + lane;
+      if (col0 + lane < N)
+        for (int r = 0; r < rows; ++r) c[(size_t)r * ldc] = stage[r * kPitch + lane];
     }
   }
 };
 
 template <int BN, class Epi>
-__global__ void __launch_bounds__(128, 1)
+__global__ void __launch_bounds__(128)
     k_gemm_tc(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, Epi epi, int K,
-              int kb_per_split, uint32_t idesc) {
+              int kb_per_split, int stages, uint32_t idesc) {
   extern __shared__ uint8_t smem_raw[];
   const int nk = (K + tc::BK - 1) / tc::BK;
   const int kb0 = blockIdx.z * kb_per_split;
   const int kb1 = min(nk, kb0 + kb_per_split);
   if (kb0 >= kb1) return;  // uniform across the CTA: this split has no k-blocks
   tc::TileMainloop<BN> ml;
-  ml.carve(smem_raw);
+  ml.carve(smem_raw, stages);
   const int m0 = blockIdx.x * tc::BM, n0 = blockIdx.y * BN;
   const uint32_t tmem = ml.setup(&tma_a, &tma_b);
   int issued = 0;
@@ -85,11 +125,16 @@ __global__ void __launch_bounds__(128, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (ml.wait_done(&g_tc_status)) {
     const uint32_t lane_base = tmem + (static_cast<uint32_t>(warp * 32) << 16);
+    // the operand tiles are free once the accumulator is complete: each warp's staging buffer
+    float* stage = reinterpret_cast<float*>(ml.tiles) + warp * 32 * Epi::kPitch;
+    static_assert(4 * 32 * Epi::kPitch * sizeof(float) <= 2 * tc::stage_bytes(BN), "two stages hold the staging");
+    const int cols = min(BN, epi.N - n0);
 #pragma unroll 1
-    for (int c = 0; c < BN; c += 16) {
-      float v[16];
-      tc::tmem_ld16(lane_base + c, v);
-      epi(m0 + warp * 32 + lane, n0 + c, v);
+    for (int c = 0; c < cols; c += 32) {
+      float a[16], b[16];
+      tc::tmem_ld16(lane_base + c, a);
+      tc::tmem_ld16(lane_base + c + 16, b);
+      epi.store(stage, m0 + warp * 32, n0 + c, lane, a, b);
     }
   }
   ml.teardown(tmem, issued, &g_tc_status);
@@ -157,9 +202,19 @@ static int launch_gemm_bn(const CUtensorMap& ta, const CUtensorMap& tb, const Ge
   if (cudaError_t e = gemm_smem_attr<BN>()) return check_cuda(e, "cudaFuncSetAttribute(gemm)");
   const int nk = (int)((K + tc::BK - 1) / tc::BK);
   const int kbps = (nk + split - 1) / split;
+  // Few k-blocks (a convolution's dcol, the first layers): the tile is its
+  // load latency and its epilogue, which need other CTAs on the SM beside it,
+  // and the full ring of stages would keep them off.  Two stages of BN = 256
+  // or three of a smaller tile leave room for two or three CTAs, within the
+  // SM's 512 TMEM columns.  With the coalesced epilogue (GemmEpilogue::store):
+  // M = 262144, N = 288, K = 64, FP32 out: 248 -> 85 us (302 MB written);
+  // M = 1048576, N = 32, K = 9, BF16 out: 178 -> 81 us.  From 17 k-blocks on
+  // the full ring hides the load latency by itself (the template search's two
+  // GEMMs, 130 k-blocks, 1024 x 36864: 1.44 ms, 1.37 ms with this epilogue).
+  const int stages = kbps > 16 ? tc::stages_for(BN) : (BN >= 256 ? 2 : std::max(2, std::min(kbps, 3)));
   const dim3 grid((unsigned)((M + tc::BM - 1) / tc::BM), (unsigned)((N + BN - 1) / BN), (unsigned)split);
-  k_gemm_tc<BN, GemmEpilogue><<<grid, 128, tc::gemm_smem_bytes(BN), stream>>>(ta, tb, epi, (int)K, kbps,
-                                                                            tc::f16_idesc(tc::BM, BN, f16 ? 0 : 1));
+  k_gemm_tc<BN, GemmEpilogue><<<grid, 128, tc::gemm_smem_bytes(BN, stages), stream>>>(
+      ta, tb, epi, (int)K, kbps, stages, tc::f16_idesc(tc::BM, BN, f16 ? 0 : 1));
   return check_cuda(cudaGetLastError(), "gemm launch");
 }
 

@@ -159,9 +159,10 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 
 __host__ __device__ constexpr int stages_for(int bn) { return bn >= 256 ? 4 : (bn >= 128 ? 5 : 6); }
 __host__ __device__ constexpr uint32_t stage_bytes(int bn) { return (BM + bn) * BK * 2; }
-__host__ __device__ constexpr size_t gemm_smem_bytes(int bn) {
-  return 1024 + static_cast<size_t>(stages_for(bn)) * stage_bytes(bn) + 256;
+__host__ __device__ constexpr size_t gemm_smem_bytes(int bn, int stages) {
+  return 1024 + static_cast<size_t>(stages) * stage_bytes(bn) + 256;
 }
+__host__ __device__ constexpr size_t gemm_smem_bytes(int bn) { return gemm_smem_bytes(bn, stages_for(bn)); }
 
 // The main loop of one 128 x BN output tile over k-blocks [kb0, kb1):
 // thread 0 of warp 0 issues the TMA loads, thread 0 of warp 1 the MMAs, and
@@ -169,27 +170,29 @@ __host__ __device__ constexpr size_t gemm_smem_bytes(int bn) {
 // the `done` barrier completes.  All four warps must call it.
 template <int BN>
 struct TileMainloop {
-  static constexpr int kStages = stages_for(BN);
   static constexpr uint32_t kABytes = BM * BK * 2;
   static constexpr uint32_t kStageBytes = stage_bytes(BN);
 
-  uint8_t* tiles;     // kStages x (A tile, B tile), 1024-byte aligned
-  uint64_t* bars;     // full[kStages], empty[kStages], done
+  int stages;         // tiles in flight
+  uint8_t* tiles;     // stages x (A tile, B tile), 1024-byte aligned
+  uint64_t* bars;     // full[stages], empty[stages], done
   uint32_t* tmem_slot;
   volatile int* abort_flag;
   int* consumed;      // k-blocks whose MMAs were issued (for the drain on abort)
 
-  __device__ void carve(uint8_t* smem_raw) {
+  // smem_raw holds gemm_smem_bytes(BN, n_stages) bytes.
+  __device__ void carve(uint8_t* smem_raw, int n_stages = stages_for(BN)) {
+    stages = n_stages;
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     tiles = base;
-    bars = reinterpret_cast<uint64_t*>(base + kStages * kStageBytes);
-    tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 1);
+    bars = reinterpret_cast<uint64_t*>(base + stages * kStageBytes);
+    tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * stages + 1);
     abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     consumed = const_cast<int*>(abort_flag) + 1;
   }
   __device__ uint32_t full(int s) const { return smem_u32(bars + s); }
-  __device__ uint32_t empty(int s) const { return smem_u32(bars + kStages + s); }
-  __device__ uint32_t done() const { return smem_u32(bars + 2 * kStages); }
+  __device__ uint32_t empty(int s) const { return smem_u32(bars + stages + s); }
+  __device__ uint32_t done() const { return smem_u32(bars + 2 * stages); }
   __device__ uint32_t a_tile(int s) const { return smem_u32(tiles + s * kStageBytes); }
   __device__ uint32_t b_tile(int s) const { return smem_u32(tiles + s * kStageBytes + kABytes); }
 
@@ -197,7 +200,7 @@ struct TileMainloop {
   __device__ uint32_t setup(const CUtensorMap* ta, const CUtensorMap* tb) {
     const int warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
-      for (int s = 0; s < kStages; ++s) {
+      for (int s = 0; s < stages; ++s) {
         mbar_init(full(s), 1);
         mbar_init(empty(s), 1);
       }
@@ -221,22 +224,24 @@ struct TileMainloop {
                       uint32_t tmem, uint32_t idesc, int* status, int* issued_out) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp == 0 && lane == 0) {
-      int issued = 0;
+      int issued = 0, s = 0;
+      uint32_t ph = 0;
       for (int kb = kb0; kb < kb1; ++kb) {
-        const int i = kb - kb0, s = i % kStages;
-        const uint32_t ph = (i / kStages) & 1;
         if (!mbar_wait(empty(s), ph ^ 1, abort_flag, status, kErrWaitEmpty)) break;
         mbar_arrive_expect_tx(full(s), kStageBytes);
         tma_load_2d(a_tile(s), ta, full(s), kb * BK, m0);
         tma_load_2d(b_tile(s), tb, full(s), kb * BK, n0);
         ++issued;
+        if (++s == stages) {
+          s = 0;
+          ph ^= 1;
+        }
       }
       *issued_out = issued;
     } else if (warp == 1 && lane == 0) {
-      int i = 0;
+      int i = 0, s = 0;
+      uint32_t ph = 0;
       for (int kb = kb0; kb < kb1; ++kb, ++i) {
-        const int s = i % kStages;
-        const uint32_t ph = (i / kStages) & 1;
         if (!mbar_wait(full(s), ph, abort_flag, status, kErrWaitFull)) break;
         tc_fence_after();
         const uint64_t da = sw128_desc(a_tile(s)), db = sw128_desc(b_tile(s));
@@ -245,6 +250,10 @@ struct TileMainloop {
           umma_f16(tmem, da + 2 * k, db + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
         umma_commit(empty(s));
         *consumed = i + 1;
+        if (++s == stages) {
+          s = 0;
+          ph ^= 1;
+        }
       }
       umma_commit(done());
     }
@@ -270,7 +279,7 @@ struct TileMainloop {
     if (*abort_flag) {
       if (warp == 0 && lane == 0) {
         for (int i = *consumed; i < issued; ++i)
-          mbar_wait(full(i % kStages), (i / kStages) & 1, nullptr, status, kErrDrain);
+          mbar_wait(full(i % stages), (i / stages) & 1, nullptr, status, kErrDrain);
       }
       if (warp == 1 && lane == 0) mbar_wait(done(), 0, nullptr, status, kErrDrain);
       __syncthreads();
