@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <mutex>
+#include <type_traits>
 
 #include "cjx_common.cuh"
 #include "cjx_profile.cuh"
@@ -336,38 +337,54 @@ __global__ void __launch_bounds__(kWarps * 32)
 // ---------------------------------------------------------------------------
 // Column adjoint (transpose of pass A's FFT + window).  g_T1 -> g_H.
 // ---------------------------------------------------------------------------
-template <int R>
-__global__ void __launch_bounds__(kWarps * 32)
+// The columns' first 256 rows are loaded before the tables are built, so that
+// the two latencies overlap, and N = 512 takes the transpose FFT of the forward
+// passes: 256 images 256^2 from N = 512 187 -> 117 us, 1024 images 192^2 from
+// N = 384 400 -> 295 us.
+__host__ __device__ inline int colfft_adj_stride(int n, int py, bool t512) {
+  const int plain = pad16(n > py ? n : py) + 1;
+  return t512 && plain < kStage512Size + 1 ? kStage512Size + 1 : plain;
+}
+
+template <int R, bool T512 = false>
+__global__ void __launch_bounds__(kWarps * 32, 4)
     k_colfft_adj(const float2* __restrict__ gt1, float2* __restrict__ gh, SliceGeom g) {
   constexpr int n = 32 * R;
   extern __shared__ float2 smem[];
   __shared__ float2 w32[32];
-  const int stride = pad16(max(n, g.py)) + 1;
+  const int stride = colfft_adj_stride(n, g.py, T512);
   float2* tab = smem;
   float2* bufs = smem + n;
   int* invy = reinterpret_cast<int*>(bufs + kWarps * stride);
+  const int j0 = blockIdx.x * kWarps;
+  const int ncols = min(kWarps, g.nxh - j0);
+  // staging: thread t moves column t % kWarps, rows t / kWarps + 32 q
+  const int sj = threadIdx.x % kWarps, sm0 = threadIdx.x / kWarps;
+  const float2* src = gt1 + (size_t)blockIdx.y * g.py * g.ld1 + j0 + sj;
+  float2 st[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    if (sj < ncols && sm0 + 32 * q < g.py) st[q] = src[(size_t)(sm0 + 32 * q) * g.ld1];
   build_reg_twiddles(tab, n);
   build_w32(w32);
   for (int q = threadIdx.x; q < n; q += blockDim.x) invy[q] = -1;
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    if (sj < ncols && sm0 + 32 * q < g.py) bufs[sj * stride + pad16(sm0 + 32 * q)] = st[q];
+  for (int m = sm0 + 256; m < g.py; m += 32)
+    if (sj < ncols) bufs[sj * stride + pad16(m)] = src[(size_t)m * g.ld1];
   __syncthreads();
   for (int m = threadIdx.x; m < g.py; m += blockDim.x) {
     const int s = win_src(m, n, g.py, g.pad_left_y);
     if (s >= 0) invy[s] = m;
-  }
-  const int j0 = blockIdx.x * kWarps;
-  const int ncols = min(kWarps, g.nxh - j0);
-  const float2* src = gt1 + (size_t)blockIdx.y * g.py * g.ld1 + j0;
-  for (int e = threadIdx.x; e < g.py * kWarps; e += blockDim.x) {
-    const int m = e / kWarps, jj = e % kWarps;
-    if (jj < ncols) bufs[jj * stride + pad16(m)] = src[(size_t)m * g.ld1 + jj];
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int j = j0 + warp;
   if (j < g.nxh) {
     float2* buf = bufs + warp * stride;
-    const LaneTwiddles lt = make_lane_twiddles(w32, lane);
-    const int bl = brev5(lane);
+    const int bl = T512 ? lane : brev5(lane);  // the transpose FFT takes natural lane order
+    auto staged = [](int i) { return T512 ? stage512(i) : pad16(i); };
     float2 y[R];
 #pragma unroll
     for (int n1 = 0; n1 < R; ++n1) {
@@ -375,16 +392,26 @@ __global__ void __launch_bounds__(kWarps * 32)
       y[n1] = (m >= 0) ? buf[pad16(m)] : make_float2(0.f, 0.f);
     }
     __syncwarp();
-    warp_fft_reg<R, -1>(y, tab, lt, lane);
+    if constexpr (T512) {
+      static_assert(R == 16, "the transpose FFT is 512-point");
+      warp_fft512_t<-1>(y, tab, w32, buf, lane);
 #pragma unroll
-    for (int k1 = 0; k1 < R; ++k1) buf[pad16(k1 + R * lane)] = y[k1];
+      for (int q = 0; q < R; ++q) buf[stage512(fft512_t_out(q, lane))] = y[q];
+    } else {
+      const LaneTwiddles lt = make_lane_twiddles(w32, lane);
+      warp_fft_reg<R, -1>(y, tab, lt, lane);
+#pragma unroll
+      for (int k1 = 0; k1 < R; ++k1) buf[pad16(k1 + R * lane)] = y[k1];
+    }
     __syncwarp();
     float2* col = gh + ((size_t)blockIdx.y * g.nxh + j) * g.ldh;
     const bool sym = (j == 0) || (j == n / 2);
-    for (int i = lane; i < n; i += 32) {
-      float2 v = buf[pad16(i)];
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const int i = 32 * q + lane;
+      float2 v = buf[staged(i)];
       if (sym) {
-        const float2 m = buf[pad16(i == 0 ? 0 : n - i)];
+        const float2 m = buf[staged(i == 0 ? 0 : n - i)];
         v = make_float2(0.5f * (v.x + m.x), 0.5f * (v.y - m.y));
       }
       col[i] = v;
@@ -517,104 +544,188 @@ __global__ void k_unbrick_add(float2* __restrict__ gg, const float2* __restrict_
   }
 }
 
-// One thread per sample of the half plane (16 x 16 samples per CTA): the
-// sample's cotangent gs = g_H, its 8 corners (read for dH/d(coordinate)),
-// the scatter of w * gs to the corners (MODE above; neighbouring samples of
-// a warp's 4 x 8 patch share most of their corners, about 3.3 samples per
-// voxel), and the CTA's share of dL/dR.  The scatter is bound by the L1 and
-// the L2's atomic units, so fewer atomic instructions and sectors is what
-// shortens it.
+// dH/d(coordinate) of an interior sample (all 8 corners in the grid, ax.i0 + 1 =
+// ax.i1 and so on): x differences and x interpolants of the four corner rows,
+// then the differences along y and z of those.
+template <typename Layout>
+__device__ __forceinline__ void interior_slopes(const float2* __restrict__ grid, const Layout& L, const AxisNodes& ax,
+                                                const AxisNodes& ay, const AxisNodes& az, float2 (&dH)[3]) {
+  float2 a[4], b[4];  // row r = 2 dz + dy: the values at x0 and x0 + 1
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int row = L.az((r >> 1) ? az.i1 : az.i0) + L.ay((r & 1) ? ay.i1 : ay.i0);
+    if constexpr (std::is_same<Layout, PairLayout>::value) {
+      const float4 q = __ldg(reinterpret_cast<const float4*>(grid) + row + L.ax(ax.i0));
+      a[r] = make_float2(q.x, q.y);
+      b[r] = make_float2(q.z, q.w);
+    } else {
+      a[r] = __ldg(grid + row + L.ax(ax.i0));
+      b[r] = __ldg(grid + row + L.ax(ax.i1));
+    }
+  }
+  float2 h[4];
+  dH[0] = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    h[r] = fma2(ax.w1, b[r], scale2(ax.w0, a[r]));
+    dH[0] = fma2(((r >> 1) ? az.w1 : az.w0) * ((r & 1) ? ay.w1 : ay.w0), csub(b[r], a[r]), dH[0]);
+  }
+  dH[1] = fma2(az.w1, csub(h[3], h[2]), scale2(az.w0, csub(h[1], h[0])));
+  dH[2] = fma2(ay.w1, csub(h[3], h[1]), scale2(ay.w0, csub(h[2], h[0])));
+}
+
+// A thread takes `steps` samples of one column (16 x 16 samples of the half
+// plane per CTA and step; scatter_steps): each sample's cotangent gs = g_H, its 8 corners
+// (read for dH/d(coordinate)), the scatter of w * gs to the corners (MODE
+// above; neighbouring samples of a warp's 4 x 8 patch share most of their
+// corners, about 3.3 samples per voxel), and at the end the CTA's share of
+// dL/dR, summed in double beyond kScatterFlush samples of a lane.
+// Bound by the L1's data stage, which the corner reads and the atomics share,
+// and by the instructions around them.  Without the grid gradient (256 images 256^2 from N = 512):
+// 595 us with one sample per thread, the general corner rule for every sample and a
+// reduction per 256 samples; 431 us now with 3 CTAs per SM (72 registers), 384
+// us with 4.  With it (1024 images 192^2 from N = 384) 2.27 ms, 2.19 ms now.
+// A second accumulator for the x-corner pairs at odd x0 (always one 16-byte
+// atomic per corner row) took 2.08 ms, less than its clearing and addition cost (0.2 ms).
 // EW: the Ewald sphere's full surface (N columns; the third coordinate
 // w = cw (u^2 + v^2) along R's third column, so dL/dR gains that column).
+constexpr int kScatterFlush = 4;
+
 template <typename Layout, int MODE, typename GL, bool EW>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
     k_scatter_slice(const float2* __restrict__ grid, const float2* __restrict__ gh,
                     const cjx_image_params* __restrict__ params, const int32_t* __restrict__ order,
-                    float2* __restrict__ grad_grid, double* __restrict__ grads, SliceGeom g, int64_t k0) {
+                    float2* __restrict__ grad_grid, double* __restrict__ grads, SliceGeom g, int64_t k0,
+                    int steps) {
   const Layout L(g.n);
   const GL G(g.n);  // the gradient array's layout: C order, or the bricked accumulator
   constexpr int NR = EW ? 9 : 6;  // dL/dR entries: columns 0 and 1 (as (row, column) pairs), then column 2
-  __shared__ float red[8][NR];
-  const int n = g.n;
+  __shared__ double red[8][NR];
+  const int n = g.n, half = n / 2;
   const int64_t k = k0 + blockIdx.z;
   const int64_t img = order ? (int64_t)order[k] : k;
   const double* Rm = params[img].rot;
   const float r00 = (float)Rm[0], r01 = (float)Rm[1];
   const float r10 = (float)Rm[3], r11 = (float)Rm[4];
   const float r20 = (float)Rm[6], r21 = (float)Rm[7];
+  float cw = 0.f, r02 = 0.f, r12 = 0.f, r22 = 0.f;
+  if constexpr (EW) {
+    cw = ewald_w(params + img, n);
+    r02 = (float)Rm[2];
+    r12 = (float)Rm[5];
+    r22 = (float)Rm[8];
+  }
   const bool wrap = !(g.flags & CJX_ZERO_FILL_NEGATIVE);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int du, dv;
   gather_lane_offsets<1>(warp, lane, du, dv);
   const int u = blockIdx.x * 16 + du;
-  const int v = blockIdx.y * 16 + dv;
-  const bool live = u < g.ncols && v < n;
+  const float2* column = gh + ((size_t)blockIdx.z * g.ncols + u) * g.ldh;
+  const float ux = (float)fft_index(u < g.ncols ? u : 0, n);
+  double total[NR];
   float gr[NR];
 #pragma unroll
-  for (int q = 0; q < NR; ++q) gr[q] = 0.f;
-  // the warp-aggregated form groups all 32 lanes, so there every lane runs the sample code (inactive
-  // lanes carry kNoKey)
-  if (MODE == kScatterWarpAgg || live) {
-    const float2 gs = live ? gh[((size_t)blockIdx.z * g.ncols + u) * g.ldh + v] : make_float2(0.f, 0.f);
-    const float ux = (float)fft_index(live ? u : 0, n), vy = (float)fft_index(live ? v : 0, n);
-    float o[3] = {fmaf(r01, vy, r00 * ux), fmaf(r11, vy, r10 * ux), fmaf(r21, vy, r20 * ux)};
-    float ew = 0.f;  // the surface's third coordinate
-    if constexpr (EW) {
-      ew = ewald_w(params + img, n) * fmaf(ux, ux, vy * vy);
-      o[0] = fmaf((float)Rm[2], ew, o[0]);
-      o[1] = fmaf((float)Rm[5], ew, o[1]);
-      o[2] = fmaf((float)Rm[8], ew, o[2]);
-    }
-    const AxisNodes ax = axis_nodes(o[0], n, wrap);
-    const AxisNodes ay = axis_nodes(o[1], n, wrap);
-    const AxisNodes az = axis_nodes(o[2], n, wrap);
-    float2 val[8];
-    load_corners<Layout>(grid, L, ax, ay, az, live, g.fill, val);
-    float dH[3][2] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};  // dH/do_axis (complex)
+  for (int q = 0; q < NR; ++q) {
+    total[q] = 0.0;
+    gr[q] = 0.f;
+  }
+#pragma unroll 1
+  for (int step = 0; step < steps; ++step) {
+    const int v0 = (blockIdx.y * steps + step) * 16;
+    if (v0 >= n) break;  // the same for the whole CTA
+    const int v = v0 + dv;
+    const bool live = u < g.ncols && v < n;
+    // the warp-aggregated form groups all 32 lanes, so there every lane runs the sample code (inactive
+    // lanes carry kNoKey)
+    if (MODE == kScatterWarpAgg || live) {
+      const float2 gs = live ? column[v] : make_float2(0.f, 0.f);
+      const float vy = (float)fft_index(live ? v : 0, n);
+      float o[3] = {fmaf(r01, vy, r00 * ux), fmaf(r11, vy, r10 * ux), fmaf(r21, vy, r20 * ux)};
+      float ew = 0.f;  // the surface's third coordinate
+      if constexpr (EW) {
+        ew = cw * fmaf(ux, ux, vy * vy);
+        o[0] = fmaf(r02, ew, o[0]);
+        o[1] = fmaf(r12, ew, o[1]);
+        o[2] = fmaf(r22, ew, o[2]);
+      }
+      AxisNodes nd[3];
+      bool interior = live;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const int dz = c >> 2, dy = (c >> 1) & 1, dx = c & 1;
-      const float wx = dx ? ax.w1 : ax.w0, wy = dy ? ay.w1 : ay.w0, wz = dz ? az.w1 : az.w0;
-      const float sx = dx ? 1.f : -1.f, sy = dy ? 1.f : -1.f, sz = dz ? 1.f : -1.f;
-      const float gwx = sx * wy * wz, gwy = sy * wx * wz, gwz = sz * wx * wy;
-      dH[0][0] += gwx * val[c].x; dH[0][1] += gwx * val[c].y;
-      dH[1][0] += gwy * val[c].x; dH[1][1] += gwy * val[c].y;
-      dH[2][0] += gwz * val[c].x; dH[2][1] += gwz * val[c].y;
-    }
-    if (grad_grid) {
-      if constexpr (MODE == kScatterWarpAgg) {
+      for (int d = 0; d < 3; ++d) {
+        const float f = floor_index(o[d], half, nd[d].i0);
+        nd[d].i1 = nd[d].i0 + 1;
+        nd[d].w1 = o[d] - f;
+        nd[d].w0 = 1.0f - nd[d].w1;
+        nd[d].v0 = nd[d].v1 = true;
+        interior = interior && (unsigned)nd[d].i0 < (unsigned)(n - 1);
+      }
+      float2 dH[3];  // dH/do_axis
+      if (interior) {
+        interior_slopes<Layout>(grid, L, nd[0], nd[1], nd[2], dH);
+        if (MODE != kScatterWarpAgg && grad_grid) scatter_rows<MODE>(grad_grid, G, nd[0], nd[1], nd[2], gs);
+      } else {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          nd[d] = axis_nodes(o[d], n, wrap);
+          dH[d] = make_float2(0.f, 0.f);
+        }
+        const AxisNodes &ax = nd[0], &ay = nd[1], &az = nd[2];
+        float2 val[8];
+        load_corners<Layout>(grid, L, ax, ay, az, live, g.fill, val);
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           const int dz = c >> 2, dy = (c >> 1) & 1, dx = c & 1;
-          const bool ok = live && (dz ? az.v1 : az.v0) && (dy ? ay.v1 : ay.v0) && (dx ? ax.v1 : ax.v0);
-          const int iz = dz ? az.i1 : az.i0, iy = dy ? ay.i1 : ay.i0, ix = dx ? ax.i1 : ax.i0;
-          const float w = ((dz ? az.w1 : az.w0) * (dy ? ay.w1 : ay.w0)) * (dx ? ax.w1 : ax.w0);
-          const unsigned key = ok ? (unsigned)((size_t)G.az(iz) + G.ay(iy) + G.ax(ix)) : kNoKey;
-          float2 c2 = make_float2(w * gs.x, w * gs.y);
-          if (peer_sum(key, c2, lane)) atomicAdd(&grad_grid[key], c2);
+          const float wx = dx ? ax.w1 : ax.w0, wy = dy ? ay.w1 : ay.w0, wz = dz ? az.w1 : az.w0;
+          dH[0] = fma2((dx ? wy : -wy) * wz, val[c], dH[0]);
+          dH[1] = fma2((dy ? wx : -wx) * wz, val[c], dH[1]);
+          dH[2] = fma2((dz ? wx : -wx) * wy, val[c], dH[2]);
         }
-      } else {
-        scatter_rows<MODE>(grad_grid, G, ax, ay, az, gs);
+        if (MODE != kScatterWarpAgg && grad_grid) scatter_rows<MODE>(grad_grid, G, ax, ay, az, gs);
+      }
+      if constexpr (MODE == kScatterWarpAgg) {
+        if (grad_grid) {
+          __syncwarp();
+          const AxisNodes &ax = nd[0], &ay = nd[1], &az = nd[2];
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const int dz = c >> 2, dy = (c >> 1) & 1, dx = c & 1;
+            const bool ok = live && (dz ? az.v1 : az.v0) && (dy ? ay.v1 : ay.v0) && (dx ? ax.v1 : ax.v0);
+            const int iz = dz ? az.i1 : az.i0, iy = dy ? ay.i1 : ay.i0, ix = dx ? ax.i1 : ax.i0;
+            const float w = ((dz ? az.w1 : az.w0) * (dy ? ay.w1 : ay.w0)) * (dx ? ax.w1 : ax.w0);
+            const unsigned key = ok ? (unsigned)((size_t)G.az(iz) + G.ay(iy) + G.ax(ix)) : kNoKey;
+            float2 c2 = make_float2(w * gs.x, w * gs.y);
+            if (peer_sum(key, c2, lane)) atomicAdd(&grad_grid[key], c2);
+          }
+        }
+      }
+      if (live) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          const float dLdo = gs.x * dH[a].x + gs.y * dH[a].y;
+          gr[2 * a] = fmaf(dLdo, ux, gr[2 * a]);
+          gr[2 * a + 1] = fmaf(dLdo, vy, gr[2 * a + 1]);
+          if constexpr (EW) gr[6 + a] = fmaf(dLdo, ew, gr[6 + a]);
+        }
       }
     }
-    if (live) {
+    if (step % kScatterFlush == kScatterFlush - 1) {
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        const float dLdo = gs.x * dH[a][0] + gs.y * dH[a][1];
-        gr[2 * a] = dLdo * ux;
-        gr[2 * a + 1] = dLdo * vy;
-        if constexpr (EW) gr[6 + a] = dLdo * ew;
+      for (int q = 0; q < NR; ++q) {
+        total[q] += (double)gr[q];
+        gr[q] = 0.f;
       }
     }
   }
 #pragma unroll
-  for (int q = 0; q < NR; ++q) gr[q] = warp_sum(gr[q]);
-  if (lane == 0)
-    for (int q = 0; q < NR; ++q) red[warp][q] = gr[q];
+  for (int q = 0; q < NR; ++q) {
+    total[q] += (double)gr[q];
+    for (int s = 16; s > 0; s >>= 1) total[q] += __shfl_xor_sync(0xffffffffu, total[q], s);
+    if (lane == 0) red[warp][q] = total[q];
+  }
   __syncthreads();
   if (threadIdx.x < NR) {
     double acc = 0.0;
-    for (int w = 0; w < 8; ++w) acc += (double)red[w][threadIdx.x];
+    for (int w = 0; w < 8; ++w) acc += red[w][threadIdx.x];
     atomicAdd(&grads[img * 16 + kGradRot + threadIdx.x], acc);
   }
 }
@@ -1291,10 +1402,11 @@ static int ensure_adjoint_smem_attrs() {
 #define CJX_ADJ_ATTR(R)                                                    \
   if (e == cudaSuccess) e = allow_smem_adj(k_colfft_loss_adj<R>);          \
   if (e == cudaSuccess) e = allow_smem_adj(k_rows_adj<R>);                 \
-  if (e == cudaSuccess) e = allow_smem_adj(k_colfft_adj<R>);
+  if (e == cudaSuccess) e = allow_smem_adj(k_colfft_adj<R, false>);
     CJX_ADJ_ATTR(1) CJX_ADJ_ATTR(2) CJX_ADJ_ATTR(3) CJX_ADJ_ATTR(4) CJX_ADJ_ATTR(5)
     CJX_ADJ_ATTR(6) CJX_ADJ_ATTR(8) CJX_ADJ_ATTR(10) CJX_ADJ_ATTR(12) CJX_ADJ_ATTR(16)
 #undef CJX_ADJ_ATTR
+    if (e == cudaSuccess) e = allow_smem_adj(k_colfft_adj<16, true>);
     if (e == cudaSuccess) e = allow_smem_adj(k_ewald_loss_adj);
     if (e == cudaSuccess) e = allow_smem_adj(k_ewald_rows_adj);
     if (e == cudaSuccess) e = allow_smem_adj(k_ewald_colfft_adj);
@@ -1315,14 +1427,23 @@ __global__ void k_zero_doubles(double* p, int64_t count) {
     p[i] = 0.0;
 }
 
+// Up to 8 steps per CTA, fewer where the tiles would not give every SM 8 CTAs.
+static int scatter_steps(dim3 tiles) {
+  const int64_t all = (int64_t)tiles.x * tiles.y * tiles.z;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(8, all / (148 * 8)));
+}
+
 template <typename Layout, typename GL, bool EW>
 static void launch_scatter(int mode, dim3 gs, cudaStream_t stream, const float2* grid, const float2* hb,
                            const cjx_image_params* params, const int32_t* order, float2* grad_grid, double* grads,
                            const SliceGeom& g, int64_t k0) {
+  const int steps = scatter_steps(gs);
+  gs.y = (gs.y + steps - 1) / steps;
   switch (mode) {
 #define CJX_SC_CASE(M)                                                                                             \
   case M:                                                                                                          \
-    k_scatter_slice<Layout, M, GL, EW><<<gs, 256, 0, stream>>>(grid, hb, params, order, grad_grid, grads, g, k0); \
+    k_scatter_slice<Layout, M, GL, EW><<<gs, 256, 0, stream>>>(grid, hb, params, order, grad_grid, grads, g, k0,   \
+                                                               steps);                                          \
     break;
     CJX_SC_CASE(kScatterCorner) CJX_SC_CASE(kScatterVec) CJX_SC_CASE(kScatterWarpAgg)
 #undef CJX_SC_CASE
@@ -1389,7 +1510,8 @@ int launch_loss_grad(const SliceGeom& g, const float2* grid, const cjx_image_par
   const size_t s_loss = sizeof(float2) * (size_t)(g.py + 2 * kWarps * (pad16(g.py) + 1));
   const size_t s_rows = sizeof(float2) * (size_t)(g.n + g.px + kWarps * (pad16(std::max(g.n, g.px)) + 1)) +
                         sizeof(int) * (size_t)g.n;
-  const size_t s_cols = sizeof(float2) * (size_t)(g.n + kWarps * (pad16(std::max(g.n, g.py)) + 1)) +
+  const bool cols_t512 = g.n == 512 && tn.fft_mode >= 3;
+  const size_t s_cols = sizeof(float2) * (size_t)(g.n + kWarps * colfft_adj_stride(g.n, g.py, cols_t512)) +
                         sizeof(int) * (size_t)g.n;
   // the Ewald row and column adjoints run on register FFTs where N and Px (rows) or N (columns) are 32 R
   const bool ew_reg_rows = ewald && tn.fft_mode >= 1 && rn && rpx;
@@ -1411,7 +1533,8 @@ int launch_loss_grad(const SliceGeom& g, const float2* grid, const cjx_image_par
   if (mode == kScatterVec && !aligned16) mode = kScatterCorner;
   // voxel grids scatter into a zeroed bricked accumulator: a warp's corner rows then touch about 12 instead of
   // about 20 distinct 128-byte lines; it is added into grid_grad (C order) at the end
-  const bool use_acc = grad_grid && acc && aligned16 && !(g.flags & CJX_GRID_SPLINE);
+  // (even N: k_unbrick_add takes x in pairs)
+  const bool use_acc = grad_grid && acc && aligned16 && !(g.flags & CJX_GRID_SPLINE) && g.n % 2 == 0;
   float2* target = use_acc ? acc : grad_grid;
   if (use_acc) {
     if (int e = check_cuda(cudaMemsetAsync(acc, 0, sizeof(float2) * bricked_elements(g.n), stream),
@@ -1488,12 +1611,16 @@ int launch_loss_grad(const SliceGeom& g, const float2* grid, const cjx_image_par
     prof_end("k_rows_adj", stream);
     prof_begin(stream);
     const dim3 gc((g.nxh + kWarps - 1) / kWarps, cnt);
-    switch (rn) {
+    if (cols_t512) {
+      k_colfft_adj<16, true><<<gc, kWarps * 32, s_cols, stream>>>(t1, hb, g);
+    } else {
+      switch (rn) {
 #define CJX_CA_CASE(R) \
   case R: k_colfft_adj<R><<<gc, kWarps * 32, s_cols, stream>>>(t1, hb, g); break;
-      CJX_CA_CASE(1) CJX_CA_CASE(2) CJX_CA_CASE(3) CJX_CA_CASE(4) CJX_CA_CASE(5)
-      CJX_CA_CASE(6) CJX_CA_CASE(8) CJX_CA_CASE(10) CJX_CA_CASE(12) CJX_CA_CASE(16)
+        CJX_CA_CASE(1) CJX_CA_CASE(2) CJX_CA_CASE(3) CJX_CA_CASE(4) CJX_CA_CASE(5)
+        CJX_CA_CASE(6) CJX_CA_CASE(8) CJX_CA_CASE(10) CJX_CA_CASE(12) CJX_CA_CASE(16)
 #undef CJX_CA_CASE
+      }
     }
     prof_end("k_colfft_adj", stream);
     }
