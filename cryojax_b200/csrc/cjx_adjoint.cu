@@ -164,14 +164,17 @@ __global__ void __launch_bounds__(kWarps * 32)
     for (int n1 = 0; n1 < R; ++n1) x[n1] = buf[pad16(32 * n1 + bl)];
     warp_fft_reg<R, -1>(x, tab, lt, lane);  // x[k1] = X[k1 + R lane]
     __syncwarp();
-#pragma unroll
-    for (int k1 = 0; k1 < R; ++k1) {
-      const int i = k1 + R * lane;
-      const EpiTerms et = epilogue_terms(i, j, py, g.px, g.flags, c, wl);
-      buf[pad16(i)] = cmul(et.mult, x[k1]);
-    }
-    __syncwarp();
     const bool self_col = (j == 0) || ((g.px % 2 == 0) && j == g.px / 2);
+    // only the Hermitian part below needs the mirrored row's value; for the other columns the multiplier is
+    // evaluated once per entry (1024 images 192^2: 441 -> 343 us)
+    if (self_col) {
+#pragma unroll
+      for (int k1 = 0; k1 < R; ++k1) {
+        const int i = k1 + R * lane;
+        buf[pad16(i)] = cmul(epilogue_terms(i, j, py, g.px, g.flags, c, wl).mult, x[k1]);
+      }
+      __syncwarp();
+    }
     const float wj = self_col ? 1.f : 2.f;
     const float inv_pp = 1.0f / ((float)py * (float)g.px);
     float2 gx[R];
@@ -179,7 +182,7 @@ __global__ void __launch_bounds__(kWarps * 32)
     for (int k1 = 0; k1 < R; ++k1) {
       const int i = k1 + R * lane;
       const EpiTerms et = epilogue_terms(i, j, py, g.px, g.flags, c, wl);
-      const float2 f = buf[pad16(i)];
+      const float2 f = cmul(et.mult, x[k1]);
       float2 fh = f;
       if (self_col) {
         const float2 fm = buf[pad16(i == 0 ? 0 : py - i)];
