@@ -239,30 +239,45 @@ __global__ void __launch_bounds__(kWarps * 32)
 // Row adjoint (transpose of pass B).  g_T2 rows -> g_T1 rows.
 // ---------------------------------------------------------------------------
 template <int RN, int RP>
-__device__ __forceinline__ void rows_pair_adj(const float2* __restrict__ gA, const float2* __restrict__ gB, bool has_b,
-                                              float2* __restrict__ outA, int ld1, float2* buf, const float2* tabN,
-                                              const float2* tabP, const LaneTwiddles& lt, int lane, const int* invx) {
+__device__ __forceinline__ void rows_pair_adj(const float2* __restrict__ gA, const float2* __restrict__ gB, bool has_a,
+                                              bool has_b, float2* __restrict__ outA, int ld1, float2* buf,
+                                              float2* tabN, float2* tabP, float2* w32, int lane, int* invx,
+                                              int pad_left) {
   constexpr int n = 32 * RN, px = 32 * RP, hp = px / 2, h = n / 2;
   const int bl = brev5(lane);
   // adjoint of r2c_Px: Z = half spectrum with interior bins halved, DC / Nyquist real
   float2 z[RP];
+  if (has_a) {  // before the tables, so that the two latencies overlap
 #pragma unroll
-  for (int n1 = 0; n1 < RP; ++n1) {
-    const int k = 32 * n1 + bl;
-    if (k == 0 || k == hp) {
-      const float2 A = gA[k];
-      const float2 B = has_b ? gB[k] : make_float2(0.f, 0.f);
-      z[n1] = make_float2(A.x, B.x);
-    } else if (k < hp) {
-      const float2 A = gA[k];
-      const float2 B = has_b ? gB[k] : make_float2(0.f, 0.f);
-      z[n1] = make_float2(0.5f * (A.x - B.y), 0.5f * (A.y + B.x));
-    } else {
-      const float2 A = gA[px - k];
-      const float2 B = has_b ? gB[px - k] : make_float2(0.f, 0.f);
-      z[n1] = make_float2(0.5f * (A.x + B.y), 0.5f * (B.x - A.y));
+    for (int n1 = 0; n1 < RP; ++n1) {
+      const int k = 32 * n1 + bl;
+      if (k == 0 || k == hp) {
+        const float2 A = gA[k];
+        const float2 B = has_b ? gB[k] : make_float2(0.f, 0.f);
+        z[n1] = make_float2(A.x, B.x);
+      } else if (k < hp) {
+        const float2 A = gA[k];
+        const float2 B = has_b ? gB[k] : make_float2(0.f, 0.f);
+        z[n1] = make_float2(0.5f * (A.x - B.y), 0.5f * (A.y + B.x));
+      } else {
+        const float2 A = gA[px - k];
+        const float2 B = has_b ? gB[px - k] : make_float2(0.f, 0.f);
+        z[n1] = make_float2(0.5f * (A.x + B.y), 0.5f * (B.x - A.y));
+      }
     }
   }
+  build_reg_twiddles(tabN, n);
+  build_reg_twiddles(tabP, px);
+  build_w32(w32);
+  for (int q = threadIdx.x; q < n; q += blockDim.x) invx[q] = -1;
+  __syncthreads();
+  for (int m = threadIdx.x; m < px; m += blockDim.x) {
+    const int s = win_src(m, n, px, pad_left);
+    if (s >= 0) invx[s] = m;
+  }
+  __syncthreads();
+  if (!has_a) return;
+  const LaneTwiddles lt = make_lane_twiddles(w32, lane);
   warp_fft_reg<RP, +1>(z, tabP, lt, lane);  // real rows a + i b (length Px)
 #pragma unroll
   for (int k1 = 0; k1 < RP; ++k1) buf[pad16(k1 + RP * lane)] = z[k1];
@@ -309,27 +324,18 @@ __global__ void __launch_bounds__(kWarps * 32)
   float2* tabP = tabN + n;
   float2* bufs = tabP + px;
   int* invx = reinterpret_cast<int*>(bufs + kWarps * stride);
-  build_reg_twiddles(tabN, n);
-  build_reg_twiddles(tabP, px);
-  build_w32(w32);
-  for (int q = threadIdx.x; q < n; q += blockDim.x) invx[q] = -1;
-  __syncthreads();
-  for (int m = threadIdx.x; m < px; m += blockDim.x) {
-    const int s = win_src(m, n, px, g.pad_left_x);
-    if (s >= 0) invx[s] = m;
-  }
-  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ra = 2 * (blockIdx.x * kWarps + warp);
-  if (ra >= g.py) return;
   const bool has_b = (ra + 1) < g.py;
   const float2* gA = gt2 + ((size_t)blockIdx.y * g.py + ra) * g.ld2;
   float2* outA = gt1 + ((size_t)blockIdx.y * g.py + ra) * g.ld1;
   float2* buf = bufs + warp * stride;
-  const LaneTwiddles lt = make_lane_twiddles(w32, lane);
   switch (rp) {
 #define CJX_RA_CASE(RPV) \
-  case RPV: rows_pair_adj<RN, RPV>(gA, gA + g.ld2, has_b, outA, g.ld1, buf, tabN, tabP, lt, lane, invx); break;
+  case RPV:                                                                                                     \
+    rows_pair_adj<RN, RPV>(gA, gA + g.ld2, ra < g.py, has_b, outA, g.ld1, buf, tabN, tabP, w32, lane, invx,     \
+                           g.pad_left_x);                                                                       \
+    break;
     CJX_RA_CASE(1) CJX_RA_CASE(2) CJX_RA_CASE(3) CJX_RA_CASE(4) CJX_RA_CASE(5)
     CJX_RA_CASE(6) CJX_RA_CASE(8) CJX_RA_CASE(10) CJX_RA_CASE(12) CJX_RA_CASE(16)
 #undef CJX_RA_CASE
