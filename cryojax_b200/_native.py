@@ -1005,8 +1005,14 @@ def _address(a) -> int:
     return a.__array_interface__["data"][0]
 
 
-def _rows(a, n: int, width: int):
-    """(array, stride in doubles) of float64 rows [width] shared by all images, or [m, ..., width] with one per image."""
+def _rows(a, n: int, width: int, what: str):
+    """(array, stride in doubles) of float64 rows [width] shared by all images, or [m, ..., width] with one per image.
+
+    The native side reads ``width`` doubles per row, so any other last axis is refused here.
+    """
+    a = np.asarray(a, np.float64)
+    if a.ndim == 0 or a.shape[-1] != width:
+        raise ValueError(f"{what} must have {width} values in its last axis, got shape {a.shape}")
     if a.ndim > 1:
         a = a.reshape(-1, width)
         if a.shape[0] == n:
@@ -1019,6 +1025,7 @@ def _rows(a, n: int, width: int):
 
 def _column(a, n: int):
     """(array, stride in doubles) of a float64 scalar shared by all images, or of one value per image."""
+    a = np.asarray(a, np.float64)
     if a.ndim == 0:
         return a, 0
     a = a.reshape(a.shape[0])
@@ -1036,7 +1043,7 @@ def pack_image_params(n: int, quaternion, offset, columns, *, normalise: bool) -
     pixel size, kilovolts and scale; then, of a transfer theory, defocus, astigmatism, angle, aberration, contrast
     ratio, phase shift; then, of an envelope, amplitude and b-factor."""
     width = offset.shape[-1]
-    kept = [_rows(quaternion, n, 4), _rows(offset, n, width)] + [_column(c, n) for c in columns]
+    kept = [_rows(quaternion, n, 4, "quaternion"), _rows(offset, n, width, "offset")] + [_column(c, n) for c in columns]
     flags = (CJX_PACK_NORMALISE if normalise else 0) | (CJX_PACK_THEORY if len(columns) > 3 else 0) | (
         CJX_PACK_ENVELOPE if len(columns) > 9 else 0)
     sources = (ctypes.c_void_p * 13)(*[_address(a) for a, _ in kept])
@@ -1048,7 +1055,9 @@ def pack_image_params(n: int, quaternion, offset, columns, *, normalise: bool) -
 
 def orientation_order(rotations, bits: int) -> np.ndarray:
     """cjx_orientation_order of float64 [n, 3, 3] rotations (or a view of them in longer rows): int32 [n]."""
-    R = rotations
+    R = np.asarray(rotations, np.float64)
+    if R.ndim != 3 or R.shape[1:] != (3, 3):
+        raise ValueError(f"rotations must have shape (n, 3, 3), got {R.shape}")
     if R.strides[-2:] != (24, 8) or R.strides[0] % 8:
         R = np.ascontiguousarray(R)
     order = np.empty(R.shape[0], np.int32)
@@ -1060,9 +1069,11 @@ def orientation_order(rotations, bits: int) -> np.ndarray:
 
 def quaternion_grad(wxyz, d_rotation) -> np.ndarray:
     """cjx_quaternion_grad: float64 [n, 4] from quaternions [n, 4] (or [1, 4]) and dL/dR [n, 3, 2 or 3]."""
-    n, _, columns = d_rotation.shape
-    q, stride = _rows(wxyz, n, 4)
-    g = np.ascontiguousarray(d_rotation)
+    g = np.ascontiguousarray(d_rotation, np.float64)
+    if g.ndim != 3 or g.shape[1] != 3:
+        raise ValueError(f"d_rotation must have shape (n, 3, 2) or (n, 3, 3), got {g.shape}")
+    n, _, columns = g.shape
+    q, stride = _rows(wxyz, n, 4, "wxyz")
     out = np.empty((n, 4), np.float64)
     _check(load_library().cjx_quaternion_grad(n, _address(q), stride, _address(g), columns, _address(out)))
     return out
