@@ -8,6 +8,7 @@ on a CUDA device.
 from __future__ import annotations
 
 import ctypes
+import operator
 import os
 import threading
 
@@ -1062,7 +1063,7 @@ def orientation_order(rotations, bits: int) -> np.ndarray:
         R = np.ascontiguousarray(R)
     order = np.empty(R.shape[0], np.int32)
     if R.shape[0]:
-        _check(load_library().cjx_orientation_order(R.shape[0], _address(R), R.strides[0] // 8, int(bits),
+        _check(load_library().cjx_orientation_order(R.shape[0], _address(R), R.strides[0] // 8, operator.index(bits),
                                                     _address(order)))
     return order
 

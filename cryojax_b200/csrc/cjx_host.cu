@@ -113,13 +113,14 @@ extern "C" int cjx_orientation_order(int64_t n_images, const double* rotations, 
                                      int32_t* order) {
   using namespace cjx;
   if (n_images < 0 || n_images > INT32_MAX) return fail(CJX_ERR_INVALID_ARGUMENT, "n_images out of range");
-  if (bits < 1 || bits > 24) return fail(CJX_ERR_INVALID_ARGUMENT, "bits must be in [1, 24]");
+  // beyond 32 bits an index needs more than 64
+  if (bits < 1 || bits > 32) return fail(CJX_ERR_INVALID_ARGUMENT, "bits must be in [1, 32]");
   if (n_images == 0) return CJX_OK;
   if (!rotations || !order) return fail(CJX_ERR_INVALID_ARGUMENT, "rotations and order must be non-NULL");
   try {
     std::vector<int64_t> key(n_images);
     std::vector<int32_t> other(n_images);
-    const double scale = (double)((1 << bits) - 1), root2 = std::sqrt(2.0);
+    const double scale = (double)((1ll << bits) - 1), root2 = std::sqrt(2.0);
     for (int64_t i = 0; i < n_images; ++i) {
       const double* R = rotations + i * stride;
       double nx = R[2], ny = R[5], nz = R[8];  // the plane's normal, sign-free
@@ -132,7 +133,10 @@ extern "C" int cjx_orientation_order(int64_t n_images, const double* rotations, 
       const double gx = clip(std::nearbyint((k * nx / root2 + 1.0) * 0.5 * scale), 0.0, scale);
       const double gy = clip(std::nearbyint((k * ny / root2 + 1.0) * 0.5 * scale), 0.0, scale);
       const uint64_t none = 1ull << 63;  // a NaN's place: no index bit set
-      key[i] = hilbert_index(gx == gx ? (uint64_t)gx : none, gy == gy ? (uint64_t)gy : none, bits);
+      // sorted as unsigned bytes below: at 32 bits, where an index fills the signed type, its sign bit is turned
+      // over so that the order stays that of signed 64-bit integers
+      key[i] = hilbert_index(gx == gx ? (uint64_t)gx : none, gy == gy ? (uint64_t)gy : none, bits) ^
+               (bits == 32 ? INT64_MIN : 0);
     }
     for (int64_t i = 0; i < n_images; ++i) order[i] = (int32_t)i;
     int32_t *from = order, *to = other.data();

@@ -672,7 +672,7 @@ CJX_API int cjx_pack_image_params(int64_t n_images, uint32_t flags, int offset_d
                                   const int64_t* strides, cjx_image_params* out);
 /* order[n_images]: the images by the Hilbert-curve index (bits per axis) of
  * their sign-free plane normal R[:, 2] in Lambert's equal-area projection,
- * ties in input order.  rotations: row-major 3 x 3 doubles, image i at
+ * ties in input order; bits in [1, 32].  rotations: row-major 3 x 3 doubles, image i at
  * stride * i doubles.                                                      */
 CJX_API int cjx_orientation_order(int64_t n_images, const double* rotations, int64_t stride, int bits,
                                   int32_t* order);
