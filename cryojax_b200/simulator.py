@@ -802,7 +802,7 @@ class AbstractImageModel:
     def _batched_fields(self):
         tt = self.transfer_theory
         pose = self.pose
-        q = pose.wxyz if type(pose) is QuaternionPose else pose.quaternion()
+        q = _arr(pose.wxyz) if type(pose) is QuaternionPose else pose.quaternion()
         fields = [q if q.ndim > 1 else None,
                   self.pose.offset_in_angstroms if self.pose.offset_in_angstroms.ndim > 1 else None,
                   self.image_config.pixel_size, self.image_config.voltage_in_kilovolts]
