@@ -1043,7 +1043,10 @@ def pack_image_params(n: int, quaternion, offset, columns, *, normalise: bool) -
     """cjx_pack_image_params: float64 [n, 32] records.  ``columns``: float64 arrays (0-d or one value per image) of
     pixel size, kilovolts and scale; then, of a transfer theory, defocus, astigmatism, angle, aberration, contrast
     ratio, phase shift; then, of an envelope, amplitude and b-factor."""
-    width = offset.shape[-1]
+    offset = np.asarray(offset, np.float64)
+    if offset.ndim and offset.shape[-1] > 3:  # x and y; a third value is a height only where it is the last
+        offset = offset[..., :2]
+    width = 3 if offset.shape[-1:] == (3,) else 2
     kept = [_rows(quaternion, n, 4, "quaternion"), _rows(offset, n, width, "offset")] + [_column(c, n) for c in columns]
     flags = (CJX_PACK_NORMALISE if normalise else 0) | (CJX_PACK_THEORY if len(columns) > 3 else 0) | (
         CJX_PACK_ENVELOPE if len(columns) > 9 else 0)
