@@ -935,9 +935,10 @@ __device__ __forceinline__ EwaldAdj ewald_epilogue_adj(float2 a, float2 b, float
 // contrast formed, the loss taken on the Hermitian part of the x = 0 and
 // Nyquist columns (what irfftn reads), and the cotangents of both T2
 // columns (inverse FFT: the adjoint of the forward FFT) written back over them.
-__global__ void __launch_bounds__(kEwAdjWarps * 32)
+template <bool PRIMES>
+__global__ void __launch_bounds__(kEwAdjWarps * 32, PRIMES ? 4 : 5)
     k_ewald_loss_adj(float2* __restrict__ t2, const float2* __restrict__ obs, const cjx_image_params* __restrict__ params,
-                     const int32_t* __restrict__ order, double* __restrict__ grads, SliceGeom g, int64_t k0,
+                     const int32_t* __restrict__ order, double* __restrict__ grads, const __grid_constant__ SliceGeom g, int64_t k0,
                      float norm) {
   extern __shared__ float2 smem[];
   __shared__ float red[kEwAdjWarps][4];
@@ -967,8 +968,8 @@ __global__ void __launch_bounds__(kEwAdjWarps * 32)
       if (pair) b[i] = col[(size_t)i * g.ld2 + xm];
     }
     __syncwarp();
-    const float2* A = warp_fft<-1>(a, a + py, g.plan_py, tw, lane);
-    const float2* B = pair ? warp_fft<-1>(b, b + py, g.plan_py, tw, lane) : A;
+    const float2* A = warp_fft<-1, PRIMES>(a, a + py, g.plan_py, tw, lane);
+    const float2* B = pair ? warp_fft<-1, PRIMES>(b, b + py, g.plan_py, tw, lane) : A;
     __syncwarp();
     for (int i = lane; i < py; i += 32) F[i] = ewald_epilogue(A[i], B[(py - i) % py], i, x, py, px, g.flags, c);
     __syncwarp();
@@ -1006,8 +1007,8 @@ __global__ void __launch_bounds__(kEwAdjWarps * 32)
       if (pair) b[i] = gB[i];
     }
     __syncwarp();
-    const float2* GA = warp_fft<+1>(a, a + py, g.plan_py, tw, lane);
-    const float2* GB = pair ? warp_fft<+1>(b, b + py, g.plan_py, tw, lane) : GA;
+    const float2* GA = warp_fft<+1, PRIMES>(a, a + py, g.plan_py, tw, lane);
+    const float2* GB = pair ? warp_fft<+1, PRIMES>(b, b + py, g.plan_py, tw, lane) : GA;
     __syncwarp();
     for (int i = lane; i < py; i += 32) {
       col[(size_t)i * g.ld2 + x] = GA[i];
@@ -1035,8 +1036,9 @@ __global__ void __launch_bounds__(kEwAdjWarps * 32)
 // Adjoint of k_ewald_rows, one warp per row: g_T2 row -> Px-point inverse
 // (adjoint of the forward FFT) -> transpose of the Px window -> N-point
 // forward FFT (adjoint of the unnormalised inverse) -> g_T1 row.
-__global__ void __launch_bounds__(kWarps * 32)
-    k_ewald_rows_adj(const float2* __restrict__ t2, float2* __restrict__ t1, SliceGeom g) {
+template <bool PRIMES>
+__global__ void __launch_bounds__(kWarps * 32, PRIMES ? 2 : 4)
+    k_ewald_rows_adj(const float2* __restrict__ t2, float2* __restrict__ t1, const __grid_constant__ SliceGeom g) {
   extern __shared__ float2 smem[];
   const int n = g.n, px = g.px;
   const int L = max(n, px);
@@ -1054,7 +1056,7 @@ __global__ void __launch_bounds__(kWarps * 32)
   const float2* row = t2 + ((size_t)blockIdx.y * g.py + r) * g.ld2;
   for (int m = lane; m < px; m += 32) a[m] = row[m];
   __syncwarp();
-  float2* w = warp_fft<+1>(a, b, g.plan_px, twp, lane);
+  float2* w = warp_fft<+1, PRIMES>(a, b, g.plan_px, twp, lane);
   float2* z = (w == a) ? b : a;
   for (int k = lane; k < n; k += 32) z[k] = make_float2(0.f, 0.f);
   __syncwarp();
@@ -1063,7 +1065,7 @@ __global__ void __launch_bounds__(kWarps * 32)
     if (src >= 0) z[src] = w[m];
   }
   __syncwarp();
-  const float2* Z = warp_fft<-1>(z, w, g.plan_n, twn, lane);
+  const float2* Z = warp_fft<-1, PRIMES>(z, w, g.plan_n, twn, lane);
   float2* dst = t1 + ((size_t)blockIdx.y * g.py + r) * g.ld1;
   for (int k = lane; k < n; k += 32) dst[k] = Z[k];
 }
@@ -1071,8 +1073,9 @@ __global__ void __launch_bounds__(kWarps * 32)
 // Adjoint of the column inverse FFT + Py window over the full surface, one
 // warp per column j in [0, N): g_T1 column -> transpose of the window ->
 // N-point forward FFT -> the surface cotangent H[j][*].
-__global__ void __launch_bounds__(kWarps * 32)
-    k_ewald_colfft_adj(const float2* __restrict__ t1, float2* __restrict__ hb, SliceGeom g) {
+template <bool PRIMES>
+__global__ void __launch_bounds__(kWarps * 32, PRIMES ? 3 : 4)
+    k_ewald_colfft_adj(const float2* __restrict__ t1, float2* __restrict__ hb, const __grid_constant__ SliceGeom g) {
   extern __shared__ float2 smem[];
   const int n = g.n;
   float2* tw = smem;
@@ -1092,7 +1095,7 @@ __global__ void __launch_bounds__(kWarps * 32)
     if (src >= 0) a[src] = col[(size_t)m * g.ld1];
   }
   __syncwarp();
-  const float2* Z = warp_fft<-1>(a, b, g.plan_n, tw, lane);
+  const float2* Z = warp_fft<-1, PRIMES>(a, b, g.plan_n, tw, lane);
   float2* dst = hb + ((size_t)blockIdx.y * g.ncols + j) * g.ldh;
   for (int k = lane; k < n; k += 32) dst[k] = Z[k];
 }
@@ -1416,9 +1419,12 @@ static int ensure_adjoint_smem_attrs() {
     CJX_ADJ_ATTR(6) CJX_ADJ_ATTR(8) CJX_ADJ_ATTR(10) CJX_ADJ_ATTR(12) CJX_ADJ_ATTR(16)
 #undef CJX_ADJ_ATTR
     if (e == cudaSuccess) e = allow_smem_adj(k_colfft_adj<16, true>);
-    if (e == cudaSuccess) e = allow_smem_adj(k_ewald_loss_adj);
-    if (e == cudaSuccess) e = allow_smem_adj(k_ewald_rows_adj);
-    if (e == cudaSuccess) e = allow_smem_adj(k_ewald_colfft_adj);
+    for (auto* k : {k_ewald_loss_adj<false>, k_ewald_loss_adj<true>})
+      if (e == cudaSuccess) e = allow_smem_adj(k);
+    for (auto* k : {k_ewald_rows_adj<false>, k_ewald_rows_adj<true>})
+      if (e == cudaSuccess) e = allow_smem_adj(k);
+    for (auto* k : {k_ewald_colfft_adj<false>, k_ewald_colfft_adj<true>})
+      if (e == cudaSuccess) e = allow_smem_adj(k);
 #define CJX_EADJ_ATTR(R)                                                         \
   if (e == cudaSuccess) e = allow_smem_adj(k_ewald_rows_adj_reg<R>);             \
   if (e == cudaSuccess) e = allow_smem_adj(k_ewald_colfft_adj_reg<R>);          \
@@ -1565,7 +1571,8 @@ int launch_loss_grad(const SliceGeom& g, const float2* grid, const cjx_image_par
 #undef CJX_ELA_CASE
         }
       } else {
-        k_ewald_loss_adj<<<dim3((g.pxh + kEwAdjWarps - 1) / kEwAdjWarps, cnt), kEwAdjWarps * 32, e_loss, stream>>>(
+        (g.plan_py.primes ? k_ewald_loss_adj<true> : k_ewald_loss_adj<false>)
+            <<<dim3((g.pxh + kEwAdjWarps - 1) / kEwAdjWarps, cnt), kEwAdjWarps * 32, e_loss, stream>>>(
             t2, obs, params, order, grads, g, k0, norm);
       }
       prof_end("k_ewald_loss_adj", stream);
@@ -1580,7 +1587,8 @@ int launch_loss_grad(const SliceGeom& g, const float2* grid, const cjx_image_par
 #undef CJX_ERA_CASE
         }
       } else {
-        k_ewald_rows_adj<<<gr, kWarps * 32, e_rows, stream>>>(t2, t1, g);
+        (g.plan_n.primes || g.plan_px.primes ? k_ewald_rows_adj<true> : k_ewald_rows_adj<false>)
+            <<<gr, kWarps * 32, e_rows, stream>>>(t2, t1, g);
       }
       prof_end("k_ewald_rows_adj", stream);
       prof_begin(stream);
@@ -1594,7 +1602,8 @@ int launch_loss_grad(const SliceGeom& g, const float2* grid, const cjx_image_par
 #undef CJX_ECA_CASE
         }
       } else {
-        k_ewald_colfft_adj<<<gc, kWarps * 32, e_cols, stream>>>(t1, hb, g);
+        (g.plan_n.primes ? k_ewald_colfft_adj<true> : k_ewald_colfft_adj<false>)<<<gc, kWarps * 32, e_cols, stream>>>(
+            t1, hb, g);
       }
       prof_end("k_ewald_colfft_adj", stream);
     } else {

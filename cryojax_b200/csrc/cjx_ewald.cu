@@ -26,8 +26,9 @@ namespace cjx {
 constexpr int kEwWarps = 4;  // warps per CTA in the column pass (two columns each)
 
 // Pass B.
-__global__ void __launch_bounds__(kWarps * 32)
-    k_ewald_rows(const float2* __restrict__ t1, float2* __restrict__ t2, SliceGeom g) {
+template <bool PRIMES>
+__global__ void __launch_bounds__(kWarps * 32, PRIMES ? 2 : 4)
+    k_ewald_rows(const float2* __restrict__ t1, float2* __restrict__ t2, const __grid_constant__ SliceGeom g) {
   extern __shared__ float2 smem[];
   const int n = g.n, px = g.px;
   const int L = max(n, px);
@@ -45,14 +46,14 @@ __global__ void __launch_bounds__(kWarps * 32)
   const float2* row = t1 + ((size_t)blockIdx.y * g.py + r) * g.ld1;
   for (int k = lane; k < n; k += 32) a[k] = row[k];
   __syncwarp();
-  float2* z = warp_fft<+1>(a, b, g.plan_n, twn, lane);
+  float2* z = warp_fft<+1, PRIMES>(a, b, g.plan_n, twn, lane);
   float2* w = (z == a) ? b : a;
   for (int m = lane; m < px; m += 32) {
     const int src = win_src(m, n, px, g.pad_left_x);
     w[m] = (src >= 0) ? z[src] : make_float2(0.f, 0.f);
   }
   __syncwarp();
-  float2* W = warp_fft<-1>(w, z, g.plan_px, twp, lane);
+  float2* W = warp_fft<-1, PRIMES>(w, z, g.plan_px, twp, lane);
   float2* dst = t2 + ((size_t)blockIdx.y * g.py + r) * g.ld2;
   for (int k = lane; k < px; k += 32) dst[k] = W[k];
 }
@@ -60,9 +61,10 @@ __global__ void __launch_bounds__(kWarps * 32)
 // Pass C.  One warp per output column x: with the CTF, x in [0, Px/2] and
 // the warp transforms columns x and (Px - x) mod Px; without it, x in
 // [0, Px) and one column.
+template <bool PRIMES>
 __global__ void __launch_bounds__(kEwWarps * 32)
     k_ewald_colfft(const float2* __restrict__ t2, const cjx_image_params* __restrict__ params,
-                   const int32_t* __restrict__ order, float2* __restrict__ out, SliceGeom g, int64_t k0,
+                   const int32_t* __restrict__ order, float2* __restrict__ out, const __grid_constant__ SliceGeom g, int64_t k0,
                    float norm) {
   extern __shared__ float2 smem[];
   const int py = g.py, px = g.px;
@@ -89,8 +91,8 @@ __global__ void __launch_bounds__(kEwWarps * 32)
     if (pair) b[i] = src[(size_t)i * g.ld2 + xm];
   }
   __syncwarp();
-  const float2* A = warp_fft<-1>(a, a + py, g.plan_py, tw, lane);
-  const float2* B = pair ? warp_fft<-1>(b, b + py, g.plan_py, tw, lane) : A;
+  const float2* A = warp_fft<-1, PRIMES>(a, a + py, g.plan_py, tw, lane);
+  const float2* B = pair ? warp_fft<-1, PRIMES>(b, b + py, g.plan_py, tw, lane) : A;
   __syncwarp();
   float2* dst = out + (size_t)img * py * pitch + x;
   for (int i = lane; i < py; i += 32) {
@@ -366,8 +368,11 @@ static int ensure_ewald_smem() {
   static PerDeviceOnce once;
   const cudaError_t err = once.run([] {
     const int kMax = 227 * 1024;
-    cudaError_t e = cudaFuncSetAttribute(k_ewald_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ewald_colfft, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
+    cudaError_t e = cudaSuccess;
+    for (auto* k : {k_ewald_rows<false>, k_ewald_rows<true>})
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
+    for (auto* k : {k_ewald_colfft<false>, k_ewald_colfft<true>})
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
     // the register kernels also hold a static 32-entry twiddle table
     const int kMaxReg = kMax - 1024;
 #define CJX_EW_ATTR(R)                                                                                        \
@@ -410,7 +415,8 @@ int launch_ewald_rows(const SliceGeom& g, const float2* t1, float2* t2, int cnt,
   } else {
     const size_t sm = ewald_rows_smem(g);
     if (sm > 227 * 1024) return fail(CJX_ERR_UNSUPPORTED, "Ewald row pass: shared memory exceeds 227 KB");
-    k_ewald_rows<<<gd, kWarps * 32, sm, stream>>>(t1, t2, g);
+    (g.plan_n.primes || g.plan_px.primes ? k_ewald_rows<true> : k_ewald_rows<false>)<<<gd, kWarps * 32, sm, stream>>>(
+        t1, t2, g);
   }
   prof_end("k_ewald_rows", stream);
   return check_cuda(cudaGetLastError(), "k_ewald_rows launch");
@@ -436,8 +442,9 @@ int launch_ewald_colfft(const SliceGeom& g, const float2* t2, const cjx_image_pa
   } else {
     const size_t sm = ewald_cols_smem(g);
     if (sm > 227 * 1024) return fail(CJX_ERR_UNSUPPORTED, "Ewald column pass: shared memory exceeds 227 KB");
-    k_ewald_colfft<<<dim3((cols + kEwWarps - 1) / kEwWarps, cnt), kEwWarps * 32, sm, stream>>>(t2, params, order,
-                                                                                                 out, g, k0, norm);
+    (g.plan_py.primes ? k_ewald_colfft<true> : k_ewald_colfft<false>)<<<dim3((cols + kEwWarps - 1) / kEwWarps, cnt),
+                                                                       kEwWarps * 32, sm, stream>>>(
+        t2, params, order, out, g, k0, norm);
   }
   prof_end("k_ewald_colfft", stream);
   return check_cuda(cudaGetLastError(), "k_ewald_colfft launch");

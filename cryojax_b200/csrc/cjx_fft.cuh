@@ -23,15 +23,23 @@ constexpr int kMaxStages = 12;  // lengths up to 1026 have at most 10 prime fact
 struct FftPlan {
   int n;
   int nstages;  // 0 only for n = 1
+  bool primes;  // a stage has a prime radix above 7 (prime_stage)
   int radix[kMaxStages];
 };
 
-// Instructions that one warp issues for a stage of radix r over n points: the
-// rounds of 32 butterflies, each with its index arithmetic, r loads, twiddles
-// and stores (about 10 per point) and the butterfly's additions and products.
+// Cost of a stage of radix r over n points for one warp: the instructions of
+// the rounds of 32 butterflies, each with its index arithmetic, r loads,
+// twiddles and stores (about 10 per point) and the butterfly's additions and
+// products, and a wait for the shared memory between two stages, which the
+// one or two rounds of a short transform do not hide.  The cheapest plans of 33
+// lengths from 20 to 360 were timed (cjx_fft_c2c, 2^23 points): with a wait of
+// 105 to 120 instructions the plan is 0.7 % slower than the fastest on average
+// and 4 % at worst, with none 3.7 % and 14 % (40 points: 5 x 2 x 4 202 us, 8 x 5
+// 186 us; 54 points: 3 x 3 x 3 x 2 171 us, 9 x 6 151 us).
+constexpr int kStageWait = 105;
 __host__ inline int fft_stage_cost(int r, int n) {
   static const int butterfly[13] = {0, 0, 4, 14, 16, 36, 42, 70, 56, 92, 100, 0, 110};
-  return ((n / r + 31) / 32) * (20 + 10 * r + butterfly[r]);
+  return kStageWait + ((n / r + 31) / 32) * (20 + 10 * r + butterfly[r]);
 }
 
 // The cheapest product of radices <= rmax that gives m; best holds the cheapest so far.
@@ -56,11 +64,13 @@ __host__ inline void fft_plan_search(int m, int rmax, int n, int cost, FftPlan& 
 // place of the two divisions per butterfly; a quadrant of twiddles evaluated
 // instead of all; image constants once per CTA; held to 64 registers for 4
 // CTAs per SM): the three resize passes 321 + 252 + 194 us before, 206 + 157 +
-// 149 us now.
+// 149 us with all of that.
 // Prime factors above 7 first, then the odd radices, then the even ones in
 // ascending order: a stage stores at stride (product of the earlier radices)
 // x its own radix, so an odd first radix keeps the first stores free of bank
 // conflicts and a later even one starts from runs of consecutive entries.
+// A plan of two stages starts with its larger radix, whose twiddles are all 1
+// there (50 points: 10 x 5 165 us, 5 x 10 181 us).
 __host__ inline FftPlan make_fft_plan(int n) {
   FftPlan p{};
   p.n = n;
@@ -71,11 +81,16 @@ __host__ inline FftPlan make_fft_plan(int n) {
   for (int f = 11; m > 1; f += 2)
     while (m % f == 0) {
       p.radix[p.nstages++] = f;
+      p.primes = true;
       m /= f;
     }
   FftPlan cur{}, best{};
   int best_cost = 1 << 30;
   fft_plan_search(smooth, 12, n, 0, cur, best, best_cost);
+  if (best.nstages == 2 && p.nstages == 0) {
+    for (int s = 0; s < 2; ++s) p.radix[p.nstages++] = best.radix[s];
+    return p;
+  }
   for (int odd = 1; odd >= 0; --odd)
     for (int s = best.nstages - 1; s >= 0; --s)
       if ((best.radix[s] & 1) == odd) p.radix[p.nstages++] = best.radix[s];
@@ -465,6 +480,7 @@ __device__ __forceinline__ void stockham_stage(const float2* __restrict__ in, fl
 //   X[q], X[p - q] = x_0 + sum_r s_r cos(2 pi r q / p) +- i sum_r d_r sin(...),
 // real factors on (p - 1) / 2 pairs: a quarter of the multiplications of the
 // direct sum.  A lane keeps Q outputs, so that each pair read serves all of them.
+// Unrolled by 4: 1021 points 1.51 ms, 1.67 ms without.
 template <int Q, int DIR>
 __device__ __forceinline__ void prime_outputs(const float2* __restrict__ in, float2* __restrict__ out, int n, int p,
                                               int Ns, const float2* tw, int lane) {
@@ -484,6 +500,7 @@ __device__ __forceinline__ void prime_outputs(const float2* __restrict__ in, flo
     }
     const float2* lo = in + j;
     const float2* hi = in + j + n;
+#pragma unroll 4
     for (int r = 1; r <= half; ++r) {
       lo += nb;
       hi -= nb;
@@ -512,8 +529,8 @@ __device__ __forceinline__ void prime_outputs(const float2* __restrict__ in, flo
 }
 
 template <int DIR>
-__device__ __noinline__ void prime_stage(float2* __restrict__ in, float2* __restrict__ out, int n, int p, int Ns,
-                                         const float2* tw, int lane) {
+__device__ __forceinline__ void prime_stage(float2* __restrict__ in, float2* __restrict__ out, int n, int p, int Ns,
+                                            const float2* tw, int lane) {
   const int nb = n / p, half = (p - 1) / 2;
   const int tstep = n / (Ns * p);
   const unsigned inv_nb = div_inverse(nb), inv_ns = div_inverse(Ns);
@@ -537,8 +554,16 @@ __device__ __noinline__ void prime_stage(float2* __restrict__ in, float2* __rest
 
 // Transform buffer `a` (length plan.n) with scratch `b`; returns the buffer
 // holding the result (a or b).  Executed by one full warp; ends with __syncwarp.
-template <int DIR>
-__device__ float2* warp_fft(float2* a, float2* b, const FftPlan& plan, const float2* tw, int lane) {
+// PRIMES: the plan may have prime stages (plan.primes).  Every kernel has an
+// instance without them for the other lengths, held to 64 registers (4 CTAs
+// per SM), one with them that may take more, and a __grid_constant__ plan, which is
+// indexed in place instead of copied to local memory.  With prime_stage as a
+// call in a single instance, 80 registers: 48 points 195 us (cjx_fft_c2c, 2^23
+// points) before prime stages existed, 208 with the
+// call, 160 now (plan included); 360 points 90, 71, 62; 101 points 630, 243, 240; 1021 points
+// 5760, 1414, 1513.  Ewald rows of 1024 images 48^2 from N = 96: 99, 109, 91.
+template <int DIR, bool PRIMES>
+__device__ __forceinline__ float2* warp_fft(float2* a, float2* b, const FftPlan& plan, const float2* tw, int lane) {
   const int n = plan.n;
   if (plan.nstages == 0) {  // n = 1
     if (lane == 0) b[0] = a[0];
@@ -559,7 +584,9 @@ __device__ float2* warp_fft(float2* a, float2* b, const FftPlan& plan, const flo
       case 9: stockham_stage<9, DIR>(a, b, n, Ns, tw, lane); break;
       case 10: stockham_stage<10, DIR>(a, b, n, Ns, tw, lane); break;
       case 12: stockham_stage<12, DIR>(a, b, n, Ns, tw, lane); break;
-      default: prime_stage<DIR>(a, b, n, R, Ns, tw, lane); break;
+      default:
+        if constexpr (PRIMES) prime_stage<DIR>(a, b, n, R, Ns, tw, lane);
+        break;
     }
     __syncwarp();
     float2* t = a;

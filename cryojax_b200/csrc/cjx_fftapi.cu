@@ -33,9 +33,9 @@ __global__ void __launch_bounds__(256) k_fft_rows_reg(const float2* __restrict__
   for (int k1 = 0; k1 < R; ++k1) dst[k1 + R * lane] = x[k1];
 }
 
-template <int DIR>
-__global__ void __launch_bounds__(256) k_fft_rows_stockham(const float2* __restrict__ in, float2* __restrict__ out,
-                                                           int64_t count, FftPlan plan) {
+template <int DIR, bool PRIMES>
+__global__ void __launch_bounds__(256, PRIMES ? 3 : 4)
+    k_fft_rows_stockham(const float2* __restrict__ in, float2* __restrict__ out, int64_t count, const __grid_constant__ FftPlan plan) {
   extern __shared__ float2 smem[];
   const int n = plan.n;
   float2* tw = smem;
@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(256) k_fft_rows_stockham(const float2* __restr
   float2* a = bufs + warp * 2 * n;
   for (int i = lane; i < n; i += 32) a[i] = in[row * n + i];
   __syncwarp();
-  float2* r = warp_fft<DIR>(a, a + n, plan, tw, lane);
+  float2* r = warp_fft<DIR, PRIMES>(a, a + n, plan, tw, lane);
   for (int i = lane; i < n; i += 32) out[row * n + i] = r[i];
 }
 
@@ -79,15 +79,14 @@ int launch_fft_rows(int n, int dir, const float2* in, float2* out, int64_t count
     default: {
       const size_t smem = sizeof(float2) * (size_t)(n + 8 * 2 * n);
       if (smem > 227 * 1024) return fail(CJX_ERR_UNSUPPORTED, "FFT length too large");
-      cudaError_t e = cudaFuncSetAttribute(dir < 0 ? k_fft_rows_stockham<-1> : k_fft_rows_stockham<+1>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-      if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute");
       const FftPlan plan = make_fft_plan(n);
+      const auto kernel =
+          dir < 0 ? (plan.primes ? k_fft_rows_stockham<-1, true> : k_fft_rows_stockham<-1, false>)
+                  : (plan.primes ? k_fft_rows_stockham<+1, true> : k_fft_rows_stockham<+1, false>);
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute");
       const int blocks = (int)((count + 7) / 8);
-      if (dir < 0)
-        k_fft_rows_stockham<-1><<<blocks, 256, smem, s>>>(in, out, count, plan);
-      else
-        k_fft_rows_stockham<+1><<<blocks, 256, smem, s>>>(in, out, count, plan);
+      kernel<<<blocks, 256, smem, s>>>(in, out, count, plan);
     }
   }
   prof_end("k_fft_rows", s);

@@ -35,8 +35,9 @@ namespace {
 inline int fft_result_offset(const FftPlan& p, int n) { return (p.nstages == 0 || (p.nstages & 1)) ? n : 0; }
 
 // Pass 1 of irfft2: column inverse FFTs of the half plane.
+template <bool PRIMES>
 __global__ void __launch_bounds__(kWarps * 32)
-    k_pp_colifft(const float2* __restrict__ in, float2* __restrict__ t, int py, int px, FftPlan plan, int res_off) {
+    k_pp_colifft(const float2* __restrict__ in, float2* __restrict__ t, int py, int px, const __grid_constant__ FftPlan plan, int res_off) {
   extern __shared__ float2 smem[];
   const int pxh = px / 2 + 1;
   const int stride = 2 * py + 2;
@@ -66,7 +67,7 @@ __global__ void __launch_bounds__(kWarps * 32)
       }
       __syncwarp();
     }
-    warp_fft<+1>(a, a + py, plan, tw, lane);
+    warp_fft<+1, PRIMES>(a, a + py, plan, tw, lane);
   }
   __syncthreads();
   float2* dst = t + (size_t)blockIdx.y * py * pxh + j0;
@@ -78,9 +79,10 @@ __global__ void __launch_bounds__(kWarps * 32)
 
 // Pass 2 of irfft2: rows (two per warp) -> fftshift -> crop -> scale (-> mask) -> float32 output,
 // plus the per-image sum and sum of squares (double) when stats != NULL.
-__global__ void __launch_bounds__(kWarps * 32)
+template <bool PRIMES>
+__global__ void __launch_bounds__(kWarps * 32, PRIMES ? 3 : 4)
     k_pp_rows_c2r(const float2* __restrict__ t, float* __restrict__ out, int py, int px, int h, int w,
-                  const float* __restrict__ mask, double* __restrict__ stats, FftPlan plan) {
+                  const float* __restrict__ mask, double* __restrict__ stats, const __grid_constant__ FftPlan plan) {
   extern __shared__ float2 smem[];
   const int pxh = px / 2 + 1;
   float2* tw = smem;
@@ -111,7 +113,7 @@ __global__ void __launch_bounds__(kWarps * 32)
     }
   }
   __syncwarp();
-  const float2* z = warp_fft<+1>(a, b, plan, tw, lane);
+  const float2* z = warp_fft<+1, PRIMES>(a, b, plan, tw, lane);
   const float scale = (float)(1.0 / ((double)py * (double)px));
   const bool fuse_mask = mask && !stats;
   float* oa = out + ((size_t)blockIdx.y * h + r0) * w;
@@ -181,8 +183,9 @@ __global__ void __launch_bounds__(256) k_pp_normalize(float* __restrict__ out, i
 }
 
 // rfft2 pass 1: rows (two per warp) of ifftshift(image) as one complex FFT, split into the half spectra.
+template <bool PRIMES>
 __global__ void __launch_bounds__(kWarps * 32)
-    k_pp_rows_r2c(const float* __restrict__ image, float2* __restrict__ out, int py, int px, FftPlan plan) {
+    k_pp_rows_r2c(const float* __restrict__ image, float2* __restrict__ out, int py, int px, const __grid_constant__ FftPlan plan) {
   extern __shared__ float2 smem[];
   const int pxh = px / 2 + 1;
   float2* tw = smem;
@@ -203,7 +206,7 @@ __global__ void __launch_bounds__(kWarps * 32)
     a[j] = make_float2(xa[c], has_b ? xb[c] : 0.f);
   }
   __syncwarp();
-  const float2* Z = warp_fft<-1>(a, b, plan, tw, lane);
+  const float2* Z = warp_fft<-1, PRIMES>(a, b, plan, tw, lane);
   float2* oa = out + ((size_t)blockIdx.y * py + ra) * pxh;
   for (int k = lane; k < pxh; k += 32) {
     const float2 Zk = Z[k];
@@ -214,8 +217,9 @@ __global__ void __launch_bounds__(kWarps * 32)
 }
 
 // rfft2 pass 2: column forward FFTs, in place (each CTA owns its columns).
+template <bool PRIMES>
 __global__ void __launch_bounds__(kWarps * 32)
-    k_pp_colfft(float2* __restrict__ data, int py, int px, FftPlan plan, int res_off) {
+    k_pp_colfft(float2* __restrict__ data, int py, int px, const __grid_constant__ FftPlan plan, int res_off) {
   extern __shared__ float2 smem[];
   const int pxh = px / 2 + 1;
   const int stride = 2 * py + 2;
@@ -231,7 +235,7 @@ __global__ void __launch_bounds__(kWarps * 32)
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp < ncols) warp_fft<-1>(bufs + warp * stride, bufs + warp * stride + py, plan, tw, lane);
+  if (warp < ncols) warp_fft<-1, PRIMES>(bufs + warp * stride, bufs + warp * stride + py, plan, tw, lane);
   __syncthreads();
   for (int e = threadIdx.x; e < py * kWarps; e += blockDim.x) {
     const int m = e / kWarps, jj = e % kWarps;
@@ -503,10 +507,12 @@ int ensure_pp_smem() {
   static PerDeviceOnce once;
   const cudaError_t e = once.run([] {
     const int kMax = 227 * 1024;
-    cudaError_t r = cudaFuncSetAttribute(k_pp_colifft, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
-    if (r == cudaSuccess) r = cudaFuncSetAttribute(k_pp_rows_c2r, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
-    if (r == cudaSuccess) r = cudaFuncSetAttribute(k_pp_rows_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
-    if (r == cudaSuccess) r = cudaFuncSetAttribute(k_pp_colfft, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
+    cudaError_t r = cudaSuccess;
+#define CJX_PP_ATTR(K)                                                                                             \
+  if (r == cudaSuccess) r = cudaFuncSetAttribute(K<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);     \
+  if (r == cudaSuccess) r = cudaFuncSetAttribute(K<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
+    CJX_PP_ATTR(k_pp_colifft) CJX_PP_ATTR(k_pp_rows_c2r) CJX_PP_ATTR(k_pp_rows_r2c) CJX_PP_ATTR(k_pp_colfft)
+#undef CJX_PP_ATTR
     return r;
   });
   return e == cudaSuccess ? CJX_OK : check_cuda(e, "cudaFuncSetAttribute (post-processing kernels)");
@@ -572,7 +578,8 @@ extern "C" int cjx_postprocess_real(int64_t n_images, int py, int px, int h, int
 #undef CJX_PPCI
       }
     } else {
-      k_pp_colifft<<<gcol, kWarps * 32, smem_cols(py), s>>>(src, t, py, px, plan_y, fft_result_offset(plan_y, py));
+      (plan_y.primes ? k_pp_colifft<true> : k_pp_colifft<false>)<<<gcol, kWarps * 32, smem_cols(py), s>>>(
+          src, t, py, px, plan_y, fft_result_offset(plan_y, py));
     }
     prof_end("k_pp_colifft", s);
     if (normalize) {
@@ -589,7 +596,8 @@ extern "C" int cjx_postprocess_real(int64_t n_images, int py, int px, int h, int
 #undef CJX_PPRC
       }
     } else {
-      k_pp_rows_c2r<<<grow, kWarps * 32, smem_rows(px), s>>>(t, dst, py, px, h, w, mask, st, plan_x);
+      (plan_x.primes ? k_pp_rows_c2r<true> : k_pp_rows_c2r<false>)<<<grow, kWarps * 32, smem_rows(px), s>>>(
+          t, dst, py, px, h, w, mask, st, plan_x);
     }
     prof_end("k_pp_rows_c2r", s);
     if (normalize) {
@@ -649,11 +657,13 @@ extern "C" int cjx_rfft2(int64_t n_images, int py, int px, const float* image, v
     const int cnt = (int)std::min<int64_t>(65535, n_images - k0);
     float2* o = static_cast<float2*>(out) + (size_t)k0 * py * pxh;
     prof_begin(s);
-    k_pp_rows_r2c<<<dim3((py + 2 * kWarps - 1) / (2 * kWarps), cnt), kWarps * 32, smem_rows(px), s>>>(
+    (plan_x.primes ? k_pp_rows_r2c<true> : k_pp_rows_r2c<false>)<<<dim3((py + 2 * kWarps - 1) / (2 * kWarps), cnt),
+                                                                   kWarps * 32, smem_rows(px), s>>>(
         image + (size_t)k0 * py * px, o, py, px, plan_x);
     prof_end("k_pp_rows_r2c", s);
     prof_begin(s);
-    k_pp_colfft<<<dim3((pxh + kWarps - 1) / kWarps, cnt), kWarps * 32, smem_cols(py), s>>>(
+    (plan_y.primes ? k_pp_colfft<true> : k_pp_colfft<false>)<<<dim3((pxh + kWarps - 1) / kWarps, cnt), kWarps * 32,
+                                                               smem_cols(py), s>>>(
         o, py, px, plan_y, fft_result_offset(plan_y, py));
     prof_end("k_pp_colfft", s);
   }

@@ -29,10 +29,10 @@ namespace cjx {
 // ---------------------------------------------------------------------------
 // Pass A
 // ---------------------------------------------------------------------------
-template <int S, typename Layout>
+template <int S, typename Layout, bool PRIMES>
 __global__ void __launch_bounds__(kWarps * 32)
     k_gather_colifft(const float2* __restrict__ grid, const cjx_image_params* __restrict__ params,
-                     const int32_t* __restrict__ order, float2* __restrict__ t1, SliceGeom g, int64_t k0) {
+                     const int32_t* __restrict__ order, float2* __restrict__ t1, const __grid_constant__ SliceGeom g, int64_t k0) {
   const Layout L(g.n);
   extern __shared__ float2 smem[];
   const int n = g.n, h = n / 2;
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(kWarps * 32)
       }
       __syncwarp();
     }
-    warp_fft<+1>(a, b, g.plan_n, tw, lane);
+    warp_fft<+1, PRIMES>(a, b, g.plan_n, tw, lane);
   }
   __syncthreads();
 
@@ -251,8 +251,9 @@ __global__ void __launch_bounds__(256, 4)
   }
 }
 
-__global__ void __launch_bounds__(kWarps * 32, 4)
-    k_colifft_window(const float2* __restrict__ hbuf, float2* __restrict__ t1, SliceGeom g) {
+template <bool PRIMES>
+__global__ void __launch_bounds__(kWarps * 32, PRIMES ? 3 : 4)
+    k_colifft_window(const float2* __restrict__ hbuf, float2* __restrict__ t1, const __grid_constant__ SliceGeom g) {
   extern __shared__ float2 smem[];
   const int n = g.n, h = n / 2;
   const int stride = 2 * n + 2;
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
       }
       __syncwarp();
     }
-    warp_fft<+1>(a, b, g.plan_n, tw, lane);
+    warp_fft<+1, PRIMES>(a, b, g.plan_n, tw, lane);
   }
   __syncthreads();
   const int res_off = (g.plan_n.nstages == 0 || (g.plan_n.nstages & 1)) ? n : 0;
@@ -298,8 +299,9 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
 // ---------------------------------------------------------------------------
 // Pass B
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kWarps * 32, 4)
-    k_rows_c2r_r2c(const float2* __restrict__ t1, float2* __restrict__ t2, SliceGeom g) {
+template <bool PRIMES>
+__global__ void __launch_bounds__(kWarps * 32, PRIMES ? 3 : 4)
+    k_rows_c2r_r2c(const float2* __restrict__ t1, float2* __restrict__ t2, const __grid_constant__ SliceGeom g) {
   extern __shared__ float2 smem[];
   const int n = g.n, px = g.px;
   const int L = max(n, px);
@@ -333,14 +335,14 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
     }
   }
   __syncwarp();
-  float2* z = warp_fft<+1>(a, b, g.plan_n, twn, lane);  // z = a_row + i b_row (real rows)
+  float2* z = warp_fft<+1, PRIMES>(a, b, g.plan_n, twn, lane);  // z = a_row + i b_row (real rows)
   float2* w = (z == a) ? b : a;
   for (int m = lane; m < px; m += 32) {
     const int src = win_src(m, n, px, g.pad_left_x);
     w[m] = (src >= 0) ? z[src] : make_float2(0.f, 0.f);
   }
   __syncwarp();
-  float2* W = warp_fft<-1>(w, z, g.plan_px, twp, lane);
+  float2* W = warp_fft<-1, PRIMES>(w, z, g.plan_px, twp, lane);
   float2* outA = t2 + ((size_t)blockIdx.y * g.py + ra) * g.ld2;
   for (int k = lane; k < g.pxh; k += 32) {
     const float2 Wk = W[k];
@@ -353,9 +355,10 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
 // ---------------------------------------------------------------------------
 // Pass C
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kWarps * 32, 4)
+template <bool PRIMES>
+__global__ void __launch_bounds__(kWarps * 32, PRIMES ? 3 : 4)
     k_colfft_epilogue(const float2* __restrict__ t2, const cjx_image_params* __restrict__ params,
-                      const int32_t* __restrict__ order, float2* __restrict__ out, SliceGeom g, int64_t k0,
+                      const int32_t* __restrict__ order, float2* __restrict__ out, const __grid_constant__ SliceGeom g, int64_t k0,
                       float norm) {
   extern __shared__ float2 smem[];
   const int py = g.py;
@@ -382,7 +385,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp < ncols) {
     float2* a = bufs + warp * stride;
-    float2* X = warp_fft<-1>(a, a + py, g.plan_py, tw, lane);
+    float2* X = warp_fft<-1, PRIMES>(a, a + py, g.plan_py, tw, lane);
     const int j = j0 + warp;
     for (int i = lane; i < py; i += 32) X[i] = apply_filter(apply_epilogue(X[i], i, j, py, g.px, g.flags, c), g, i, j, g.pxh);
   }
@@ -893,15 +896,19 @@ static cudaError_t allow_smem(K kernel) {
 static int ensure_smem_attrs() {
   static PerDeviceOnce once;
   const cudaError_t e = once.run([] {
-    cudaError_t e = allow_smem(k_gather_colifft<1, LinearLayout>);
-    if (e == cudaSuccess) e = allow_smem(k_gather_colifft<2, LinearLayout>);
-    if (e == cudaSuccess) e = allow_smem(k_gather_colifft<4, LinearLayout>);
-    if (e == cudaSuccess) e = allow_smem(k_gather_colifft<1, BrickLayout>);
-    if (e == cudaSuccess) e = allow_smem(k_gather_colifft<2, BrickLayout>);
-    if (e == cudaSuccess) e = allow_smem(k_gather_colifft<4, BrickLayout>);
-    if (e == cudaSuccess) e = allow_smem(k_colifft_window);
-    if (e == cudaSuccess) e = allow_smem(k_rows_c2r_r2c);
-    if (e == cudaSuccess) e = allow_smem(k_colfft_epilogue);
+    cudaError_t e = cudaSuccess;
+#define CJX_SMEM_ATTR(P)                                                             \
+  if (e == cudaSuccess) e = allow_smem(k_gather_colifft<1, LinearLayout, P>);        \
+  if (e == cudaSuccess) e = allow_smem(k_gather_colifft<2, LinearLayout, P>);        \
+  if (e == cudaSuccess) e = allow_smem(k_gather_colifft<4, LinearLayout, P>);        \
+  if (e == cudaSuccess) e = allow_smem(k_gather_colifft<1, BrickLayout, P>);         \
+  if (e == cudaSuccess) e = allow_smem(k_gather_colifft<2, BrickLayout, P>);         \
+  if (e == cudaSuccess) e = allow_smem(k_gather_colifft<4, BrickLayout, P>);         \
+  if (e == cudaSuccess) e = allow_smem(k_colifft_window<P>);                         \
+  if (e == cudaSuccess) e = allow_smem(k_rows_c2r_r2c<P>);                           \
+  if (e == cudaSuccess) e = allow_smem(k_colfft_epilogue<P>);
+    CJX_SMEM_ATTR(false) CJX_SMEM_ATTR(true)
+#undef CJX_SMEM_ATTR
     return e;
   });
   return e == cudaSuccess ? CJX_OK : check_cuda(e, "cudaFuncSetAttribute (slice kernels)");
@@ -988,7 +995,8 @@ static int launch_front(const SliceGeom& g, const float2* grid, const cjx_image_
 #undef CJX_A_CASE
         }
       } else {
-        k_colifft_window<<<gc, kWarps * 32, sa, stream>>>(hb, t1, g);
+        (g.plan_n.primes ? k_colifft_window<true> : k_colifft_window<false>)<<<gc, kWarps * 32, sa, stream>>>(hb, t1,
+                                                                                                             g);
       }
       prof_end("k_colifft_window", stream);
     } else {
@@ -997,9 +1005,11 @@ static int launch_front(const SliceGeom& g, const float2* grid, const cjx_image_
       const bool bricked = (g.flags & CJX_GRID_BRICKED) != 0;
 #define CJX_GC(S)                                                                                     \
   if (bricked)                                                                                        \
-    k_gather_colifft<S, BrickLayout><<<ga, kWarps * 32, sa, stream>>>(grid, params, order, t1, g, k0); \
+    (g.plan_n.primes ? k_gather_colifft<S, BrickLayout, true> : k_gather_colifft<S, BrickLayout, false>)     \
+        <<<ga, kWarps * 32, sa, stream>>>(grid, params, order, t1, g, k0);                              \
   else                                                                                                \
-    k_gather_colifft<S, LinearLayout><<<ga, kWarps * 32, sa, stream>>>(grid, params, order, t1, g, k0);
+    (g.plan_n.primes ? k_gather_colifft<S, LinearLayout, true> : k_gather_colifft<S, LinearLayout, false>)   \
+        <<<ga, kWarps * 32, sa, stream>>>(grid, params, order, t1, g, k0);
       if (ilp == 4) {
         CJX_GC(4)
       } else if (ilp == 2) {
@@ -1038,7 +1048,8 @@ static int launch_rows(const SliceGeom& g, const float2* t1, float2* t2, int cnt
 #undef CJX_B_CASE
       }
     } else {
-      k_rows_c2r_r2c<<<gb, kWarps * 32, sb, stream>>>(t1, t2, g);
+      (g.plan_n.primes || g.plan_px.primes ? k_rows_c2r_r2c<true> : k_rows_c2r_r2c<false>)<<<gb, kWarps * 32, sb,
+                                                                                           stream>>>(t1, t2, g);
     }
     prof_end("k_rows_c2r_r2c", stream);
   return check_cuda(cudaGetLastError(), "forward launch");
@@ -1079,7 +1090,8 @@ static int launch_tail(const SliceGeom& g, const float2* t2, const cjx_image_par
 #undef CJX_C_CASE
     }
   } else {
-    k_colfft_epilogue<<<gcc, kWarps * 32, sc, stream>>>(t2, params, order, out, g, k0, norm);
+    (g.plan_py.primes ? k_colfft_epilogue<true> : k_colfft_epilogue<false>)<<<gcc, kWarps * 32, sc, stream>>>(
+        t2, params, order, out, g, k0, norm);
   }
   prof_end("k_colfft_epilogue", stream);
   return check_cuda(cudaGetLastError(), "forward launch");
