@@ -101,17 +101,19 @@ __device__ __forceinline__ void gather_colifft_body(const float2* __restrict__ g
       r22 = (float)Rm[8];
     }
     float2* col = tile + du * stride;
-    // every lane samples (columns past the edge repeat column 0, rows past N low frequencies); only the stores
-    // are guarded.  The row index and its signed frequency are carried in floating point (exact): with the
+    // Every lane samples (columns past the edge repeat column 0); only the stores are guarded.  Rows past N, the
+    // last iteration's second sample where R is odd, are not sampled: 1562 images 80^2 from N = 160 259 us with
+    // them, 240 without (247 before the rest of this), 4096 images 48^2 from N = 96 269, 251 (267).  Guarding the
+    // columns past the edge as well takes 1 % longer.  The row index and its signed frequency are carried in floating point (exact): with the
     // floor by addition (floor_index) and the one-permute Morton index, 2.90 -> 2.83 ms per 2048 images 320^2.
-    bool act[S];
-#pragma unroll
-    for (int s = 0; s < S; ++s) act[s] = true;
     float row = (float)dv;
 #pragma unroll 1
     for (int p0 = 0; p0 < R; p0 += S, row += 32.0f * S) {
       float ox[S], oy[S], oz[S];
       float2 val[S];
+      bool act[S];
+#pragma unroll
+      for (int s = 0; s < S; ++s) act[s] = R % S == 0 || p0 + s < R;
 #pragma unroll
       for (int s = 0; s < S; ++s) {
         const float v = row + 32.0f * s;
