@@ -181,14 +181,26 @@ __global__ void __launch_bounds__(256, (kGatherCtas<S, Layout>))
 // CTAs per SM 3.30, 2.70, 2.48 and 2.98 ms (5 spill).  A warp takes 4 columns x 8 rows as four groups of 2 x 4 samples;
 // the four lanes of a team then exchange their shares, so that lane t ends
 // with the sample of group t, and store it.
-// CTA patch: 16 columns x 16 kSplineSteps rows.
+// CTA patch: 16 columns x 16 steps rows: up to kSplineSteps steps, fewer where
+// the tiles would not give every SM its 4 CTAs (spline_steps).  A warp of
+// columns past the plane has nothing to do and returns.  With 4 steps always
+// and those warps sampling: one image 320^2 from N = 512 22 us, 14 now (17 with
+// a lane per sample), 2048 images 32^2 from N = 64 248 and 204 (360).
 constexpr int kSplineSteps = 4;
+
+static int spline_steps(dim3 tiles) {
+  const int64_t all = (int64_t)tiles.x * tiles.y * tiles.z;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(kSplineSteps, all / (148 * 4)));
+}
 
 __global__ void __launch_bounds__(256, 4)
     k_gather_spline_team(const float4* __restrict__ coef, const cjx_image_params* __restrict__ params,
-                         const int32_t* __restrict__ order, float2* __restrict__ hbuf, SliceGeom g, int64_t k0) {
+                         const int32_t* __restrict__ order, float2* __restrict__ hbuf, SliceGeom g, int64_t k0,
+                         int steps) {
   const SplinePairLayout L(g.n);
   const int n = g.n;
+  const int u0 = blockIdx.x * 16 + 4 * ((threadIdx.x >> 5) & 3);
+  if (u0 >= g.ncols) return;  // the same for the whole warp; no barrier below
   const int64_t k = k0 + blockIdx.z;
   const int64_t img = order ? (int64_t)order[k] : k;
   const double* R = params[img].rot;
@@ -207,21 +219,21 @@ __global__ void __launch_bounds__(256, 4)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = lane & 3, ly = t & 1, lz = t >> 1;
   const int su = (lane >> 2) & 1, sv = lane >> 3;
-  const int u0 = blockIdx.x * 16 + 4 * (warp & 3);
   float ux[2], bx[2], by[2], bz[2];  // the two columns this lane samples
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
-    ux[c] = (float)fft_index(min(u0 + 2 * c + su, n - 1), n);
+    ux[c] = (float)fft_index(min(u0 + 2 * c + su, g.ncols - 1), n);
     bx[c] = r00 * ux[c];
     by[c] = r10 * ux[c];
     bz[c] = r20 * ux[c];
   }
 #pragma unroll 1
-  for (int step = 0; step < kSplineSteps; ++step) {
-    const int v0 = (blockIdx.y * kSplineSteps + step) * 16 + 8 * (warp >> 2);
+  for (int step = 0; step < steps; ++step) {
+    const int v0 = (blockIdx.y * steps + step) * 16 + 8 * (warp >> 2);
     if (v0 >= n) break;  // the same for the whole warp
     float2 p[4];
-    // every lane samples (columns and rows past the edge repeat others); only the stores are guarded
+    // every lane samples (columns past the edge repeat the last, rows past N are low frequencies); only the stores
+    // are guarded
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int c = q & 1;
@@ -970,8 +982,11 @@ static int launch_front(const SliceGeom& g, const float2* grid, const cjx_image_
     CJX_GSM(S, 0)       \
   }
       if (spline && pairs) {
-        const dim3 gt((g.ncols + 15) / 16, (g.n + 16 * kSplineSteps - 1) / (16 * kSplineSteps), cnt);
-        k_gather_spline_team<<<gt, 256, 0, stream>>>(reinterpret_cast<const float4*>(grid), params, order, hb, g, k0);
+        dim3 gt((g.ncols + 15) / 16, (g.n + 15) / 16, cnt);
+        const int steps = spline_steps(gt);
+        gt.y = (gt.y + steps - 1) / steps;
+        k_gather_spline_team<<<gt, 256, 0, stream>>>(reinterpret_cast<const float4*>(grid), params, order, hb, g, k0,
+                                                     steps);
       } else if (ilp == 4) {
         CJX_GS(4)
       } else if (ilp == 2) {
