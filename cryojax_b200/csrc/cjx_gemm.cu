@@ -202,17 +202,26 @@ static int launch_gemm_bn(const CUtensorMap& ta, const CUtensorMap& tb, const Ge
   if (cudaError_t e = gemm_smem_attr<BN>()) return check_cuda(e, "cudaFuncSetAttribute(gemm)");
   const int nk = (int)((K + tc::BK - 1) / tc::BK);
   const int kbps = (nk + split - 1) / split;
-  // Few k-blocks (a convolution's dcol, the first layers): the tile is its
-  // load latency and its epilogue, which need other CTAs on the SM beside it,
-  // and the full ring of stages would keep them off.  Two stages of BN = 256
+  const dim3 grid((unsigned)((M + tc::BM - 1) / tc::BM), (unsigned)((N + BN - 1) / BN), (unsigned)split);
+  // Where the grid gives every SM one CTA at most, the tile has the full ring
+  // of stages to itself (all 16 k-blocks of M = 1024, N = 4096, K = 1024, 128
+  // CTAs of BN = 256: 14.2 us with two stages, 11.9 with four; before the
+  // coalesced epilogue 15.8).
+  // More CTAs than that and few k-blocks (a convolution's dcol, the first
+  // layers): the tile is its load latency and its epilogue, which need other
+  // CTAs on the SM beside it, and the full ring would keep them off.  Two stages of BN = 256
   // or three of a smaller tile leave room for two or three CTAs, within the
   // SM's 512 TMEM columns.  With the coalesced epilogue (GemmEpilogue::store):
   // M = 262144, N = 288, K = 64, FP32 out: 248 -> 85 us (302 MB written);
-  // M = 1048576, N = 32, K = 9, BF16 out: 178 -> 81 us.  From 17 k-blocks on
-  // the full ring hides the load latency by itself (the template search's two
-  // GEMMs, 130 k-blocks, 1024 x 36864: 1.44 ms, 1.37 ms with this epilogue).
-  const int stages = kbps > 16 ? tc::stages_for(BN) : (BN >= 256 ? 2 : std::max(2, std::min(kbps, 3)));
-  const dim3 grid((unsigned)((M + tc::BM - 1) / tc::BM), (unsigned)((N + BN - 1) / BN), (unsigned)split);
+  // M = 1048576, N = 32, K = 9, BF16 out: 178 -> 81 us; M = 4096, N = 4096, K =
+  // 1024 57 -> 37 us.
+  // From 17 k-blocks on the full ring (M = N = 4096, K = 1088: 58 -> 48 us; the template search's two
+  // GEMMs, 130 k-blocks, 1024 x 36864: 1.44 ms, 1.37 ms with this epilogue).  Two stages are faster there
+  // for BN = 256 (39 us at K = 1088) and slower for the smaller tiles (M = N = 512, K = 2048: 14.7 -> 17.3 us).
+  const bool alone = (int64_t)grid.x * grid.y * grid.z <= 148;
+  const int stages = kbps > 16 ? tc::stages_for(BN)
+                     : alone   ? std::min(tc::stages_for(BN), std::max(2, kbps))
+                               : (BN >= 256 ? 2 : std::max(2, std::min(kbps, 3)));
   k_gemm_tc<BN, GemmEpilogue><<<grid, 128, tc::gemm_smem_bytes(BN, stages), stream>>>(
       ta, tb, epi, (int)K, kbps, stages, tc::f16_idesc(tc::BM, BN, f16 ? 0 : 1));
   return check_cuda(cudaGetLastError(), "gemm launch");
