@@ -346,19 +346,22 @@ __global__ void __launch_bounds__(kWarps * 32)
 // ---------------------------------------------------------------------------
 // Column adjoint (transpose of pass A's FFT + window).  g_T1 -> g_H.
 // ---------------------------------------------------------------------------
-// The columns' first 256 rows are loaded before the tables are built, so that
-// the two latencies overlap, and N = 512 takes the transpose FFT of the forward
-// passes: 256 images 256^2 from N = 512 187 -> 117 us, 1024 images 192^2 from
-// N = 384 400 -> 295 us.
+// The columns' first rows, N of them but 256 at most, are loaded before the
+// tables are built, so that the two latencies overlap, and N = 512 takes the
+// transpose FFT of the forward passes: 256 images 256^2 from N = 512 187 -> 117
+// us, 1024 images 192^2 from N = 384 400 -> 295 us.  Short columns need few
+// registers for that (40 to R = 5, 6 CTAs per SM): 2048 images 32^2 from N = 64 33
+// us (33 with late loads; 44 with 256 rows' registers and 4 CTAs), 64^2 from
+// N = 128 82 us (93; 99).
 __host__ __device__ inline int colfft_adj_stride(int n, int py, bool t512) {
   const int plain = pad16(n > py ? n : py) + 1;
   return t512 && plain < kStage512Size + 1 ? kStage512Size + 1 : plain;
 }
 
 template <int R, bool T512 = false>
-__global__ void __launch_bounds__(kWarps * 32, 4)
+__global__ void __launch_bounds__(kWarps * 32, R <= 5 ? 6 : 4)
     k_colfft_adj(const float2* __restrict__ gt1, float2* __restrict__ gh, SliceGeom g) {
-  constexpr int n = 32 * R;
+  constexpr int n = 32 * R, kEarly = R < 8 ? R : 8;
   extern __shared__ float2 smem[];
   __shared__ float2 w32[32];
   const int stride = colfft_adj_stride(n, g.py, T512);
@@ -370,17 +373,17 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
   // staging: thread t moves column t % kWarps, rows t / kWarps + 32 q
   const int sj = threadIdx.x % kWarps, sm0 = threadIdx.x / kWarps;
   const float2* src = gt1 + (size_t)blockIdx.y * g.py * g.ld1 + j0 + sj;
-  float2 st[8];
+  float2 st[kEarly];
 #pragma unroll
-  for (int q = 0; q < 8; ++q)
+  for (int q = 0; q < kEarly; ++q)
     if (sj < ncols && sm0 + 32 * q < g.py) st[q] = src[(size_t)(sm0 + 32 * q) * g.ld1];
   build_reg_twiddles(tab, n);
   build_w32(w32);
   for (int q = threadIdx.x; q < n; q += blockDim.x) invy[q] = -1;
 #pragma unroll
-  for (int q = 0; q < 8; ++q)
+  for (int q = 0; q < kEarly; ++q)
     if (sj < ncols && sm0 + 32 * q < g.py) bufs[sj * stride + pad16(sm0 + 32 * q)] = st[q];
-  for (int m = sm0 + 256; m < g.py; m += 32)
+  for (int m = sm0 + 32 * kEarly; m < g.py; m += 32)
     if (sj < ncols) bufs[sj * stride + pad16(m)] = src[(size_t)m * g.ld1];
   __syncthreads();
   for (int m = threadIdx.x; m < g.py; m += blockDim.x) {
