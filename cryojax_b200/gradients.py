@@ -151,12 +151,14 @@ def squared_residual_and_grad(model, observed, *, grid_grad: bool = True, observ
         raise NotImplementedError("the loss gradient needs padded_shape == shape")
     vol = model.volume_parametrization.get_representation()
     integ = model.volume_integrator
-    obs_f = observed if observed_is_fourier else observed_to_fourier(observed)  # runs while the host packs
     params = model.image_params()
     n = params.shape[0]
     ewald = not integ.is_projection_approximation  # EwaldSphereExtraction: R's third column enters too
     dev = vol.device
     flags = model._flags() | integ._base_flags()
+    # what the model refuses is refused above, before any device work; the transform runs while the host sorts
+    obs_f = observed if observed_is_fourier else observed_to_fourier(observed)
+    host_order = orientation_order(params[:, 0:9].reshape(-1, 3, 3)) if sort_orientations else None
     if hasattr(vol, "spline_coefficients"):  # gradient with respect to the spline coefficients
         grid, grad_shape = vol.spline_coefficients, tuple(vol.spline_coefficients.shape)
         flags |= nat.CJX_GRID_SPLINE
@@ -177,9 +179,7 @@ def squared_residual_and_grad(model, observed, *, grid_grad: bool = True, observ
     if tuple(obs_f.shape) != (n, py, px // 2 + 1):
         raise ValueError(f"observed has shape {tuple(obs_f.shape)}, expected {(n, py, px // 2 + 1)} in Fourier space")
     pd = torch.as_tensor(params, device=dev)
-    order = None
-    if sort_orientations:
-        order = torch.as_tensor(orientation_order(params[:, 0:9].reshape(-1, 3, 3)), device=dev)
+    order = None if host_order is None else torch.as_tensor(host_order, device=dev)
     grads = torch.empty((n, nat.GRAD_DOUBLES), dtype=torch.float64, device=dev)
     gg = torch.zeros(grad_shape, dtype=torch.complex64, device=dev) if grid_grad else None
     ws = torch.empty(max(nat.loss_workspace_size(desc, n), 1), dtype=torch.uint8, device=dev)
