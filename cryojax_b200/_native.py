@@ -1006,12 +1006,20 @@ def _address(a) -> int:
     return a.__array_interface__["data"][0]
 
 
+_FLOAT64 = np.dtype(np.float64)
+
+
+def _doubles(a):
+    """a as a float64 array (itself if it is one: one of these per parameter and call)."""
+    return a if type(a) is np.ndarray and a.dtype is _FLOAT64 else np.asarray(a, np.float64)
+
+
 def _rows(a, n: int, width: int, what: str):
     """(array, stride in doubles) of float64 rows [width] shared by all images, or [m, ..., width] with one per image.
 
     The native side reads ``width`` doubles per row, so any other last axis is refused here.
     """
-    a = np.asarray(a, np.float64)
+    a = _doubles(a)
     if a.ndim == 0 or a.shape[-1] != width:
         raise ValueError(f"{what} must have {width} values in its last axis, got shape {a.shape}")
     if a.ndim > 1:
@@ -1026,7 +1034,7 @@ def _rows(a, n: int, width: int, what: str):
 
 def _column(a, n: int):
     """(array, stride in doubles) of a float64 scalar shared by all images, or of one value per image."""
-    a = np.asarray(a, np.float64)
+    a = _doubles(a)
     if a.ndim == 0:
         return a, 0
     a = a.reshape(a.shape[0])
@@ -1043,10 +1051,12 @@ def pack_image_params(n: int, quaternion, offset, columns, *, normalise: bool) -
     """cjx_pack_image_params: float64 [n, 32] records.  ``columns``: float64 arrays (0-d or one value per image) of
     pixel size, kilovolts and scale; then, of a transfer theory, defocus, astigmatism, angle, aberration, contrast
     ratio, phase shift; then, of an envelope, amplitude and b-factor."""
-    offset = np.asarray(offset, np.float64)
-    if offset.ndim and offset.shape[-1] > 3:  # x and y; a third value is a height only where it is the last
-        offset = offset[..., :2]
-    width = 3 if offset.shape[-1:] == (3,) else 2
+    offset = _doubles(offset)
+    width = offset.shape[-1] if offset.ndim else 0
+    if width > 3:  # x and y; a third value is a height only where it is the last
+        offset, width = offset[..., :2], 2
+    elif width < 2:
+        raise ValueError(f"offset must have 2 or 3 values in its last axis, got shape {offset.shape}")
     kept = [_rows(quaternion, n, 4, "quaternion"), _rows(offset, n, width, "offset")] + [_column(c, n) for c in columns]
     flags = (CJX_PACK_NORMALISE if normalise else 0) | (CJX_PACK_THEORY if len(columns) > 3 else 0) | (
         CJX_PACK_ENVELOPE if len(columns) > 9 else 0)
