@@ -453,7 +453,6 @@ __global__ void __launch_bounds__(kWarps * 32)
       x[n1] = v;
     }
   }
-  for (int m = threadIdx.x; m < g.py; m += blockDim.x) winy[m] = win_src(m, n, g.py, g.pad_left_y);
   __syncthreads();
   if (j < g.ncols) {
     const LaneTwiddles lt = make_lane_twiddles(w32, lane);
@@ -468,6 +467,9 @@ __global__ void __launch_bounds__(kWarps * 32)
       for (int k1 = 0; k1 < R; ++k1) buf[pad16(k1 + R * lane)] = x[k1];
     }
   }
+  // the window's map last: its place among the loads decided the pass's time (1024 images 320^2 from N = 512: 490
+  // us there with divisions in win_src, 508 without, 492 here; 8192 images 64^2 from N = 128 286, 278, 273)
+  for (int m = threadIdx.x; m < g.py; m += blockDim.x) winy[m] = win_src(m, n, g.py, g.pad_left_y);
   __syncthreads();
   const int ncols = min(kWarps, g.ncols - j0);
   float2* dst = t1 + (size_t)blockIdx.y * g.py * g.ld1 + j0;
