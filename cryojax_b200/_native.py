@@ -1007,10 +1007,11 @@ def _address(a) -> int:
 
 
 _FLOAT64 = np.dtype(np.float64)
+_SOURCES, _STRIDES = ctypes.c_void_p * 13, ctypes.c_int64 * 13  # cjx_pack_image_params' sources
 
 
 def _doubles(a):
-    """a as a float64 array (itself if it is one: one of these per parameter and call)."""
+    """a as a float64 array (itself if it is one)."""
     return a if type(a) is np.ndarray and a.dtype is _FLOAT64 else np.asarray(a, np.float64)
 
 
@@ -1034,8 +1035,9 @@ def _rows(a, n: int, width: int, what: str):
 
 def _column(a, n: int):
     """(array, stride in doubles) of a float64 scalar shared by all images, or of one value per image."""
-    a = _doubles(a)
-    if a.ndim == 0:
+    if type(a) is not np.ndarray or a.dtype is not _FLOAT64:
+        a = np.asarray(a, np.float64)
+    if not a.shape:
         return a, 0
     a = a.reshape(a.shape[0])
     if a.shape[0] != n:
@@ -1060,8 +1062,8 @@ def pack_image_params(n: int, quaternion, offset, columns, *, normalise: bool) -
     kept = [_rows(quaternion, n, 4, "quaternion"), _rows(offset, n, width, "offset")] + [_column(c, n) for c in columns]
     flags = (CJX_PACK_NORMALISE if normalise else 0) | (CJX_PACK_THEORY if len(columns) > 3 else 0) | (
         CJX_PACK_ENVELOPE if len(columns) > 9 else 0)
-    sources = (ctypes.c_void_p * 13)(*[_address(a) for a, _ in kept])
-    strides = (ctypes.c_int64 * 13)(*[s for _, s in kept])
+    sources = _SOURCES(*[a.__array_interface__["data"][0] for a, _ in kept])
+    strides = _STRIDES(*[s for _, s in kept])
     out = np.empty((n, PARAMS_DOUBLES), np.float64)
     _check(load_library().cjx_pack_image_params(n, flags, width, sources, strides, _address(out)))
     return out
