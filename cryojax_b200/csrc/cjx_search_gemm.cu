@@ -308,25 +308,31 @@ __global__ void k_ncc_argmax(const float* __restrict__ num, const float* __restr
 // scores at a time with the list's last entry: after the first few hundred
 // templates hardly any passes (about m ln(T / 8 m) insertions per warp in all),
 // so the pass runs at the speed of reading num and den once.  A list per
-// thread made almost every step of a warp wait for some lane's insertion:
-// 0.64 ms for 1024 rows of 36,864 templates, 0.15 ms now (0.05 ms to read
-// the 302 MB).
+// thread made almost every step of a warp wait for some lane's insertion: 1024
+// rows of 36,864 templates, m = 8, 0.67 ms, 0.12 ms now (0.05 ms to read the
+// 302 MB), and 0.58 and 0.27 ms where the scores rise from the first template to
+// the last, the order with the most insertions (1.92 ms while the lowest of a
+// warp's candidates went first).
 
 __device__ __forceinline__ bool key_gt(float a, int32_t ia, float b, int32_t ib) {
   return a > b || (a == b && ia < ib);
 }
 
-// Inserts the candidates (s, t) of the lanes in `want` into the warp's sorted
-// list (v, ix: entry k in lane k < m); `last` is entry m - 1.  Called by whole
-// warps.
+// Inserts the candidates (s, t) of the lanes in `want`, each above the list's
+// last entry, into the warp's sorted list (v, ix: entry k in lane k < m);
+// `last` is entry m - 1.  The best goes first, so that of 32 rising scores only
+// m are inserted.  Called by whole warps.
 __device__ __forceinline__ void list_insert(unsigned want, float s, int32_t t, float& v, int32_t& ix, float& last_v,
                                             int32_t& last_i, int m, int lane) {
   while (want) {
-    const int src = __ffs((int)want) - 1;
-    want &= want - 1u;
+    int src = __ffs((int)want) - 1;
+    if (want & (want - 1u)) {
+      const unsigned bits = __float_as_uint(s);
+      const unsigned rank = (want >> lane & 1u) ? ((bits >> 31) ? ~bits : bits | 0x80000000u) : 0u;  // ordered as s
+      src = __ffs((int)__ballot_sync(0xffffffffu, rank == __reduce_max_sync(0xffffffffu, rank))) - 1;
+    }
     const float cs = __shfl_sync(0xffffffffu, s, src);
     const int32_t ci = __shfl_sync(0xffffffffu, t, src);
-    if (!key_gt(cs, ci, last_v, last_i)) continue;  // an earlier lane's insertion may have raised the bar
     const int pos = __popc(__ballot_sync(0xffffffffu, lane < m && key_gt(v, ix, cs, ci)));
     const float up_v = __shfl_up_sync(0xffffffffu, v, 1);
     const int32_t up_i = __shfl_up_sync(0xffffffffu, ix, 1);
@@ -339,6 +345,7 @@ __device__ __forceinline__ void list_insert(unsigned want, float s, int32_t t, f
     }
     last_v = __shfl_sync(0xffffffffu, v, m - 1);
     last_i = __shfl_sync(0xffffffffu, ix, m - 1);
+    want = __ballot_sync(0xffffffffu, (want >> lane & 1u) && lane != src && key_gt(s, t, last_v, last_i));
   }
 }
 
@@ -366,7 +373,7 @@ __global__ void __launch_bounds__(256)
       d[q] = t < T ? drow[t] : 0.f;
     }
 #pragma unroll
-    for (int q = 0; q < kTopUnroll; ++q) {
+    for (int q = kTopUnroll - 1; q >= 0; --q) {  // last group first: of rising scores the others are then not inserted
       const int64_t t = t0 + 32 * q + lane;
       const float nq = n[q] * yr, dq = d[q] * zr;
       const float s = (dq > 0.f && o2 > 0.f) ? nq * rsqrtf(dq * o2) : 0.f;
