@@ -962,9 +962,9 @@ def measure_spline(dev, grid, batch, cfg, steps, warmup, n_images, cpu_images):
     res = {"value": n_images / (ms / 1000.0), "unit": UNIT, "images": n_images, "ms_per_step": ms,
            "layout": "x-pair bricked coefficients, side N + 2 = %d" % (n + 2),
            "coefficients_ms": coef_ms,
-           "gather_us_per_image": prof["k_gather_slice"][1] * 1000.0 / n_images,
+           "gather_us_per_image": prof["k_gather_spline_team"][1] * 1000.0 / n_images,
            "kernels_per_step": {k: {"launches": c, "ms": t} for k, (c, t) in prof.items()},
-           "bound": "L1 data-stage wavefronts (ncu: 83 % of peak; DRAM 27 %)"}
+           "bound": "L1 data-stage wavefronts (ncu: 80 % of peak; issue slots 65 %, DRAM 33 %)"}
     got = out[:PARITY_IMAGES].cpu().numpy()
     del out, wsf, pd
     if cpu_images:

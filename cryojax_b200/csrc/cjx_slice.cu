@@ -175,8 +175,8 @@ __global__ void __launch_bounds__(256, (kGatherCtas<S, Layout>))
 }
 
 // The split gather for spline coefficients in the x-pair layout, four lanes
-// per sample (sample_spline_team4), bound by the L1's data stage (77 % of its
-// wavefronts, ncu) next to the issue slots (65 %).  512 images 320^2 from
+// per sample (sample_spline_team4), bound by the L1's data stage (80 % of its
+// wavefronts, ncu, 64 images) next to the issue slots (65 %).  512 images 320^2 from
 // N = 512: 3.13 ms with a lane per sample, 2.48 ms now; with 2, 3, 4 and 5
 // CTAs per SM 3.30, 2.70, 2.48 and 2.98 ms (5 spill).  A warp takes 4 columns x 8 rows as four groups of 2 x 4 samples;
 // the four lanes of a team then exchange their shares, so that lane t ends
@@ -998,7 +998,7 @@ static int launch_front(const SliceGeom& g, const float2* grid, const cjx_image_
       }
 #undef CJX_GS
 #undef CJX_GSM
-      prof_end("k_gather_slice", stream);
+      prof_end(spline && pairs ? "k_gather_spline_team" : "k_gather_slice", stream);
       prof_begin(stream);
       const dim3 gc((g.ncols + kWarps - 1) / kWarps, cnt);
       if (fast && t512) {
