@@ -1446,16 +1446,24 @@ __global__ void k_zero_doubles(double* p, int64_t count) {
 }
 
 // Up to 8 steps per CTA, fewer where the tiles would not give every SM 8 CTAs.
-static int scatter_steps(dim3 tiles) {
-  const int64_t all = (int64_t)tiles.x * tiles.y * tiles.z;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(8, all / (148 * 8)));
+// With the volume's gradient a step is long and so is the last wave's tail: 4
+// steps at most until every SM has 32 CTAs of 8 (64 images 160^2 115 us before
+// there were steps, 121 with 8 steps, 115 with 4; 1024 images 192^2 2284, 2184,
+// 2203), and a quarter of the steps with warp-aggregated atomics, which take more
+// than twice the time (64 images 160^2 246 us, 289 with 8 steps, 262 with 4, 250 with 2).
+// Without it the reduction counts more (62 us with 2 steps, 52 with 8).
+static int scatter_steps(dim3 tiles, bool volume_gradient, int mode) {
+  const int per_sm = volume_gradient && mode == kScatterWarpAgg ? 32 : 8;
+  const int64_t per_slot = (int64_t)tiles.x * tiles.y * tiles.z / (148 * per_sm);
+  const int64_t most = volume_gradient && per_slot < 32 ? 4 : 8;
+  return (int)std::max<int64_t>(1, std::min(most, per_slot));
 }
 
 template <typename Layout, typename GL, bool EW>
 static void launch_scatter(int mode, dim3 gs, cudaStream_t stream, const float2* grid, const float2* hb,
                            const cjx_image_params* params, const int32_t* order, float2* grad_grid, double* grads,
                            const SliceGeom& g, int64_t k0) {
-  const int steps = scatter_steps(gs);
+  const int steps = scatter_steps(gs, grad_grid != nullptr, mode);
   gs.y = (gs.y + steps - 1) / steps;
   switch (mode) {
 #define CJX_SC_CASE(M)                                                                                             \

@@ -1,8 +1,8 @@
 """GPU: the scatter with several steps per CTA and several CTAs per column of tiles, the last of them partial.
 
 The number of steps grows with the batch (up to 8; one per CTA in the small batches that the large one is compared
-with).  N = 192 has 12 row tiles: 3 steps give 4 CTAs, 5 steps 3 with a partial last one and a sum flushed twice, 8
-steps 2.  dL/dR sums 192 x 97 (slice) or 192 x 192 (Ewald) signed terms, at most four of a lane in single precision:
+with; with the volume's gradient 4 until the batch is four times as large).  N = 192 has 12 row tiles: 3 steps give 4
+CTAs, 4 steps 3, 5 steps 3 with a partial last one and a sum flushed twice, 8 steps 2.  dL/dR sums 192 x 97 (slice) or 192 x 192 (Ewald) signed terms, at most four of a lane in single precision:
 3 x 2^-24 of the terms' sizes, about sqrt(36864) = 192 times their sum: 3.5e-5, bound 5e-5 of the batch's largest.  The
 volume's gradient is a single-precision sum in no fixed order: relative L2 2e-5.
 """
@@ -27,8 +27,9 @@ def test_large_batch_matches_small_batches(cuda_device, surface, mode, steps):
     from cryojax_b200.gradients import squared_residual_and_grad
 
     column_tiles = ROW_TILES if surface == "ewald" else (BOX + 1 + 15) // 16
-    n = -(-steps * 148 * 8 // (ROW_TILES * column_tiles))
-    assert n * ROW_TILES * column_tiles // (148 * 8) == steps or steps == 8
+    tiles_per_slot = 32 if steps == 8 and mode is not None else steps
+    n = -(-tiles_per_slot * 148 * 8 // (ROW_TILES * column_tiles))
+    assert n * ROW_TILES * column_tiles // (148 * 8) == tiles_per_slot
     rng = np.random.default_rng(steps)
     torch.manual_seed(steps)
     vol = S.FourierVoxelGridVolume(torch.randn(2 * BOX, 2 * BOX, 2 * BOX, dtype=torch.complex64, device="cuda"))
