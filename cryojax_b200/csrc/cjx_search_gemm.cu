@@ -72,8 +72,6 @@ __global__ void k_pack_templates(const float2* __restrict__ img, int py, int px,
   }
 }
 
-// Per observed image (block): Y16 = (w conj(m) O) / yinv, Z16 = (w |m|^2) / zinv
-// with yinv, zinv the rows' RMS, and oo = sum w |O|^2.
 // Row i and column j of entry e = thread + 256 k of a [py][pxh] image, carried
 // from one entry of a thread to its next.
 struct EntryWalk {
@@ -96,6 +94,8 @@ struct EntryWalk {
 
 constexpr size_t kPackCacheBytes = 72 * 1024;
 
+// Per observed image (block): Y16 = (w conj(m) O) / yinv, Z16 = (w |m|^2) / zinv
+// with yinv, zinv the rows' RMS, and oo = sum w |O|^2.
 // Bound by the instructions of the multipliers.  CACHE: the second pass reads
 // them from shared memory (8 bytes per entry) instead of evaluating them again;
 // with the image's constants once per CTA and the entry's row and column carried:
@@ -629,7 +629,7 @@ int cjx_pack_observed(const void* observed, const cjx_image_params* params, int6
   if (!observed || !params || !y16 || !z16 || !oo || !yinv || !zinv)
     return cjx::fail(CJX_ERR_INVALID_ARGUMENT, "pack_observed: NULL pointer");
   if (n > 2147483647LL) return cjx::fail(CJX_ERR_UNSUPPORTED, "pack_observed: too many images");
-  // up to 72 KB of multipliers (sides to 132), 3 CTAs per SM; beyond that they are evaluated twice
+  // up to 72 KB of multipliers (sides to 135), 3 CTAs per SM; beyond that they are evaluated twice
   const size_t smem = sizeof(float2) * (size_t)py * (px / 2 + 1);
   const bool cache = smem <= cjx::kPackCacheBytes;
   if (cache) {

@@ -436,7 +436,9 @@ CJX_API int cjx_rfft2(int64_t n_images, int py, int px, const float* image, void
  * corner lands on the same voxel sum their contributions with warp shuffles
  * and one lane per voxel issues the atomic.
  * CJX_TUNE_SPLINE_ILP: samples per lane in the cubic-spline gather
- * (CJX_GRID_SPLINE; 1, 2 or 4, default 4).                                 */
+ * (CJX_GRID_SPLINE; 1, 2 or 4, default 4).  It and CJX_TUNE_GATHER_TILE have
+ * no effect on coefficients in the x-pair layout (CJX_GRID_BRICKED_PAIRS),
+ * whose gather spreads each sample over four lanes of a fixed patch.       */
 #define CJX_TUNE_GATHER_ILP 1
 #define CJX_TUNE_CHUNK_BYTES 2
 #define CJX_TUNE_GATHER_MODE 3
