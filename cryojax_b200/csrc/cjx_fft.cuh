@@ -546,7 +546,11 @@ __device__ __forceinline__ void prime_stage(float2* __restrict__ in, float2* __r
     in[j + (p - r) * nb] = csub(a, b);
   }
   __syncwarp();
-  if (nb * (half / 4 + 1) >= 20)  // enough lanes busy with four outputs each
+  // Rounds of 32 lanes: four outputs each take three times as long as one.  2^23 points with one, with four: 101
+  // points 237 us, 309 (2 rounds, 1); 163 points 314, 309 (3, 1); 202 points 207, 184 (4, 1); 262 points 240, 287 (5,
+  // 2); 340 points 98, 92 (6, 2); 676 points 117, 110 (12, 4).  Of 60 lengths the slower one is chosen at four, by
+  // at most 6 %.
+  if (3 * ((nb * (half / 4 + 1) + 31) / 32) <= (nb * (half + 1) + 31) / 32)
     prime_outputs<4, DIR>(in, out, n, p, Ns, tw, lane);
   else
     prime_outputs<1, DIR>(in, out, n, p, Ns, tw, lane);
