@@ -1040,7 +1040,7 @@ __global__ void __launch_bounds__(kEwAdjWarps * 32, PRIMES ? 4 : 5)
 // (adjoint of the forward FFT) -> transpose of the Px window -> N-point
 // forward FFT (adjoint of the unnormalised inverse) -> g_T1 row.
 template <bool PRIMES>
-__global__ void __launch_bounds__(kWarps * 32, PRIMES ? 2 : 4)
+__global__ void __launch_bounds__(kWarps * 32, PRIMES ? 3 : 4)
     k_ewald_rows_adj(const float2* __restrict__ t2, float2* __restrict__ t1, const __grid_constant__ SliceGeom g) {
   extern __shared__ float2 smem[];
   const int n = g.n, px = g.px;

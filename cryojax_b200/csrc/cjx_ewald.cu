@@ -25,9 +25,11 @@ namespace cjx {
 
 constexpr int kEwWarps = 4;  // warps per CTA in the column pass (two columns each)
 
-// Pass B.
+// Pass B.  The instance with prime stages takes 80 registers (3 CTAs per SM): at 117 (2) images of sides to 250
+// from twice that are slower (725 images 83^2 371 us, 345 at 80) and larger ones, where shared memory keeps CTAs
+// off anyway, faster (19 images 509^2 1.16 ms, 1.33 at 80).
 template <bool PRIMES>
-__global__ void __launch_bounds__(kWarps * 32, PRIMES ? 2 : 4)
+__global__ void __launch_bounds__(kWarps * 32, PRIMES ? 3 : 4)
     k_ewald_rows(const float2* __restrict__ t1, float2* __restrict__ t2, const __grid_constant__ SliceGeom g) {
   extern __shared__ float2 smem[];
   const int n = g.n, px = g.px;
